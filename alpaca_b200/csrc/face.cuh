@@ -26,6 +26,39 @@ __host__ __device__ constexpr bool left_nonzero(int n, int l) {
 }
 
 
+// Fast-build FP64 forms of the per-state quantities, with the kinetic energy
+// as a plain chain of products.
+
+// A reconstructed state's 1/rho, principal velocity and pressure.
+struct ReconState {
+  double one, v, p;
+};
+template <int DIM, int DIR>
+__device__ __forceinline__ ReconState recon_state(Eos const &e, double const (&c)[DIM + 2]) {
+  double q = c[MOMX] * c[MOMX];
+  if constexpr (DIM > 1) q = fma(c[MOMX + 1], c[MOMX + 1], q);
+  if constexpr (DIM > 2) q = fma(c[MOMX + 2], c[MOMX + 2], q);
+  ReconState s;
+  s.one = inv(c[MASS]);
+  s.v = c[MOMX + DIR] * s.one;
+  double const one = e.safe && !(c[MASS] > DBL_EPSILON) ? 1.0 / DBL_EPSILON : s.one;
+  s.p = fma(e.gamma - 1.0, fma(-0.5 * one, q, c[ENERGY]), -(e.gamma * e.B));
+  if (e.safe) s.p = dmax(s.p, -e.B + DBL_EPSILON);
+  return s;
+}
+
+// Physical flux of a cell along DIR.
+template <int DIM, int DIR>
+__device__ __forceinline__ void phys_flux(Eos const &e, double const (&c)[DIM + 2],
+                                          double (&f)[DIM + 2]) {
+  ReconState const s = recon_state<DIM, DIR>(e, c);
+  f[MASS] = c[MOMX + DIR];
+  f[ENERGY] = (c[ENERGY] + s.p) * s.v;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d)
+    f[MOMX + d] = d == DIR ? fma(c[MOMX + d], s.v, s.p) : c[MOMX + d] * s.v;
+}
+
 // Flux of one face from its 6-cell stencil (the reference's per-face work:
 // FiniteVolumeScheme::ComputeFluxes<DIR> with the selected reconstruction and
 // HLLC, or FluxSplittingScheme::ComputeFluxes<DIR>). Writes the flux in double
@@ -45,6 +78,85 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
   constexpr int C = W / 2 - 1;  // the face's left cell i in the stencil
 
   if constexpr (SCHEME == FV_CHAR || SCHEME == FS_ROE) {
+    if constexpr (ALP_FAST && sizeof(T) == 8 && P::is_default) {
+      // the factored characteristic frame on the five differences of the six
+      // cells (each side's reconstruction is its own cell plus an increment)
+      auto const ct = char_cell<DIM, DIR>(eos, cons[C]);
+      auto const cn = char_cell<DIM, DIR>(eos, cons[C + 1]);
+      if (!(cons[C][MASS] > 0.0) || !(cons[C + 1][MASS] > 0.0)) valid = false;
+      auto const r = char_frame<DIM, DIR>(eos, ct, cn, cons[C][MASS], cons[C + 1][MASS]);
+      if constexpr (SCHEME == FV_CHAR) {
+        double G[NE][5];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          double x[NE], ch[NE];
+#pragma unroll
+          for (int l = 0; l < NE; ++l) x[l] = cons[m + 1][l] - cons[m][l];
+          char_project<DIM, DIR>(r, x, ch);
+#pragma unroll
+          for (int n = 0; n < NE; ++n) G[n][m] = ch[n];
+        }
+        double il[NE], ir[NE];
+#pragma unroll
+        for (int n = 0; n < NE; ++n) weno5_increments(G[n], char_eps<DIM>(r, n), il[n], ir[n]);
+        double cm[NE], cp[NE];
+        char_restore<DIM, DIR>(r, cons[C], il, 1.0, cm);
+        char_restore<DIM, DIR>(r, cons[C + 1], ir, -1.0, cp);
+        if (!(cm[MASS] > DBL_EPSILON) || !(cp[MASS] > DBL_EPSILON)) valid = false;
+        auto const sm = recon_state<DIM, DIR>(eos, cm);
+        auto const sp = recon_state<DIM, DIR>(eos, cp);
+        if (!(sm.p > -B) || !(sp.p > -B)) valid = false;
+        hllc<DIM, DIR, double>(eos, cm, cp, sm.p, sp.p, sm.v, sp.v, sm.one, sp.one, fd);
+      } else {
+        // Roe flux-vector splitting: the split fluxes f +/- alpha u of each
+        // wave from the projected differences of f and u. The mean of the two
+        // reconstructions is (f_i + f_i+1) / 2 plus R times half of
+        // (left increment - right increment - alpha L (u_i+1 - u_i)).
+        double const al[3] = {fabs(r.up - r.c), fabs(r.up), fabs(r.up + r.c)};
+        double A[NE][5], N[NE][5], w[NE];
+        double fa[NE], fb[NE], fi[NE];
+        phys_flux<DIM, DIR>(eos, cons[0], fa);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          double x[NE], y[NE], cu[NE], cf[NE];
+          if (m == 2) {
+#pragma unroll
+            for (int l = 0; l < NE; ++l) fi[l] = fa[l];
+          }
+          phys_flux<DIM, DIR>(eos, cons[m + 1], fb);
+#pragma unroll
+          for (int l = 0; l < NE; ++l) {
+            x[l] = cons[m + 1][l] - cons[m][l];
+            y[l] = fb[l] - fa[l];
+          }
+          if (m == 2) {
+#pragma unroll
+            for (int l = 0; l < NE; ++l) fi[l] = 0.5 * (fi[l] + fb[l]);
+          }
+          char_project<DIM, DIR>(r, x, cu);
+          char_project<DIM, DIR>(r, y, cf);
+#pragma unroll
+          for (int n = 0; n < NE; ++n) {
+            double const a = n == 0 ? al[0] : (n == NE - 1 ? al[2] : al[1]);
+            if (m < 4) A[n][m] = fma(a, cu[n], cf[n]);
+            if (m > 0) N[n][m] = fma(-a, cu[n], cf[n]);
+            if (m == 2) w[n] = a * cu[n];
+          }
+#pragma unroll
+          for (int l = 0; l < NE; ++l) fa[l] = fb[l];
+        }
+#pragma unroll
+        for (int n = 0; n < NE; ++n) {
+          double l, q;
+          A[n][4] = 0.0;
+          N[n][0] = 0.0;
+          weno5_increments_two(A[n], N[n], char_eps<DIM>(r, n), l, q);
+          w[n] = 0.5 * ((l - q) - w[n]);
+        }
+        char_restore<DIM, DIR>(r, fi, w, 1.0, fd);
+      }
+      return valid;
+    }
     auto const pt = cell_prims<DIM, DIR>(eos, cons[C]);
     auto const pn = cell_prims<DIM, DIR>(eos, cons[C + 1]);
     if (!(pt.rho > 0.0) || !(pn.rho > 0.0)) valid = false;
@@ -270,6 +382,23 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
     double prim[W][NE];
 #pragma unroll
     for (int m = 0; m < W; ++m) {
+      if constexpr (ALP_FAST && P::is_default) {
+        // velocities, then the pressure with the kinetic energy u . m / 2
+        prim[m][RHO] = cons[m][MASS];
+        double const one = inv(cons[m][MASS]);
+        double um = 0.0;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          prim[m][VELX + d] = cons[m][MOMX + d] * one;
+          um = d == 0 ? prim[m][VELX] * cons[m][MOMX]
+                      : fma(prim[m][VELX + d], cons[m][MOMX + d], um);
+        }
+        if (eos.safe && !(cons[m][MASS] > DBL_EPSILON)) um *= cons[m][MASS] * (1.0 / DBL_EPSILON);
+        double p = fma(eos.gamma - 1.0, fma(-0.5, um, cons[m][ENERGY]), -(eos.gamma * eos.B));
+        if (eos.safe) p = dmax(p, -eos.B + DBL_EPSILON);
+        prim[m][PRES] = p;
+        continue;
+      }
       prim[m][RHO] = cons[m][MASS];
       double const one_rho = inv(cons[m][MASS]);
 #pragma unroll
@@ -316,6 +445,25 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
 #pragma unroll
         for (int m = 0; m < W; ++m) arr[m] = T(prim[m][n]);
         pol.pair(arr, pm[n], pp[n]);
+      }
+      if constexpr (ALP_FAST && sizeof(T) == 8 && P::is_default) {
+        // the upwind side's conservatives alone (hllc_upwind)
+        if (!(pm[RHO] > DBL_EPSILON) || !(pp[RHO] > DBL_EPSILON)) valid = false;
+        if (!(pm[PRES] > -B) || !(pp[PRES] > -B)) valid = false;
+        HllcUpwind const h = hllc_upwind(eos, pm[RHO], pp[RHO], pm[PRES], pp[PRES],
+                                         pm[VELX + DIR], pp[VELX + DIR], inv(pm[RHO]),
+                                         inv(pp[RHO]));
+        fd[MASS] = h.rho * h.k;
+        double q = 0.0;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          double const v = h.right ? pp[VELX + d] : pm[VELX + d];
+          q = d == 0 ? v * v : fma(v, v, q);
+          fd[MOMX + d] = d == DIR ? fma(h.rho, h.g, h.p) : v * fd[MASS];
+        }
+        double const E = fma(0.5 * h.rho, q, (h.p + eos.gamma * eos.B) * inv(eos.gamma - 1.0));
+        fd[ENERGY] = fma(E, h.k, h.pe);
+        return valid;
       }
       // PrimeStatesToConservatives (prime_state_handler.h:195-275)
       T cm[NE], cp[NE];

@@ -28,31 +28,26 @@
 
 namespace alp {
 
-// Reciprocal by Newton-Raphson iteration on f(y) = 1/y - b (y <- y + y(1 - b y)),
-// seeded with the PTX approximate reciprocal; two iterations take the seed's
-// ~2^-20 relative error below one ulp.
+// Reciprocal by one third-order Householder iteration on f(y) = 1/y - b
+// (Householder 1970: y <- y (1 + e + e^2), e = 1 - b y), seeded with the PTX
+// approximate reciprocal: the seed's ~2^-20 relative error becomes its cube,
+// 2^-60, in three operations (two Newton steps: four).
 __device__ __forceinline__ double rcp_nr(double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  double e = fma(-b, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-b, y, 1.0);
-  y = fma(y, e, y);
-  return y;
+  double const e = fma(-b, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
-// 1/sqrt(x) by Newton-Raphson iteration on f(y) = 1/y^2 - x
-// (y <- y + y (1 - x y^2) / 2), seeded with the PTX approximate reciprocal
-// square root; each iteration squares the relative error, two take it below
-// the rounding of the last steps (fast build only).
+// 1/sqrt(x) by one third-order Householder iteration on f(y) = 1/y^2 - x
+// (y <- y (1 + e/2 + 3 e^2/8), e = 1 - x y^2), seeded with the PTX approximate
+// reciprocal square root (fast build only); the remaining error is 5/16 e^3,
+// below 2^-58.
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x * y, y, 1.0);
-  y = fma(0.5 * y, e, y);
-  e = fma(-x * y, y, 1.0);
-  y = fma(0.5 * y, e, y);
-  return y;
+  double const e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // 1/x: IEEE division in the strict build, rcp_nr (double) or the PTX
@@ -248,66 +243,66 @@ template <typename T> __device__ __forceinline__ T weno5_right(T const (&a)[6]) 
 }
 
 // Fast-build WENO5-JS from first differences. For a stencil v1..v5 around
-// the face of v3, with g1..g4 = v2-v1, v3-v2, v4-v3, v5-v4 and the second
-// differences d1..d3 = g2-g1, g3-g2, g4-g3, the three candidate values are
-//   q1 = v3 + (5 g2 - 2 g1) / 6, q2 = v3 + (g2 + 2 g3) / 6, q3 = v3 + (4 g3 - g4) / 6
-// and the smoothness indicators, four times larger with eps four times larger
-// (every (beta + eps)^2 scaled alike, so the weights do not change),
-//   13/3 d_k^2 + e_k^2 with e = 3 g2 - g1, g2 + g3, g4 - 3 g3.
-// The ideal weights 0.1, 0.6, 0.3 enter as 1, 6, 3. The result is
-// v3 + num / (6 den); passing the differences of the mirrored stencil without
-// their sign change (g_k' = -g) negates num and leaves den unchanged.
-// alpha_k scaled by t1 t2 t3 (no reciprocal here). In float the t_k are first
-// multiplied by the power of two that brings the largest into [1, 2) (exact:
-// the scale is built from the exponent bits), so the products stay inside the
-// float range; a product that underflows belongs to a weight below 2^-126 of
-// the largest.
-template <typename T> struct Weno5Frac { T num, den; };
+// the face of v3, with g1..g4 = v2-v1, v3-v2, v4-v3, v5-v4, the second
+// differences d1..d3 = g2-g1, g3-g2, g4-g3, a = g2 + d1 and b = g3 - d3, the
+// three candidate values are
+//   q1 = v3 + (2 a + g2) / 6, q2 = v3 + (2 g3 + g2) / 6, q3 = v3 + (2 g3 + b) / 6
+// and the reference's smoothness indicators 13/12 (..)^2 + 1/4 (..)^2 become
+//   4/3 d1^2 + g2 a, 4/3 d2^2 + g2 g3, 4/3 d3^2 + g3 b
+// (in each the terms' absolute sum stays below twice the indicator, so no
+// digits are lost to cancellation). q_k = 4/3 d_k^2 + eps is passed in: the two
+// sides of a face share two of them. With t_k the squared indicators (eps
+// added) and the ideal weights 0.1, 0.6, 0.3 as 1, 6, 3, scaled by t1 t2 t3,
+// the result is v3 + num / (6 den). The differences of the mirrored stencil,
+// reversed without their sign change, negate num and leave den unchanged.
+// 20 operations a side; with the indicators as two squares each it took 26.
+struct Weno5Frac { double num, den; };
 
-template <typename T>
-__device__ __forceinline__ Weno5Frac<T> weno5_frac(T g1, T g2, T g3, T g4, T d1, T d2, T d3) {
-  T const c = T(13.0 / 3.0);
-  T const e1 = T(3.0) * g2 - g1;
-  T const e2 = g2 + g3;
-  T const e3 = g4 + T(-3.0) * g3;
-  T const eps = T(4.0e-6);
-  T const s1 = (c * d1) * d1 + (e1 * e1 + eps);
-  T const s2 = (c * d2) * d2 + (e2 * e2 + eps);
-  T const s3 = (c * d3) * d3 + (e3 * e3 + eps);
-  T const t1 = s1 * s1, t2 = s2 * s2, t3 = s3 * s3;
-  T const r1 = T(5.0) * g2 + T(-2.0) * g1;
-  T const r2 = g2 + T(2.0) * g3;
-  T const r3 = T(4.0) * g3 - g4;
-  T u1 = t1, u2 = t2, u3 = t3;
-  if constexpr (sizeof(T) == 4) {
-    unsigned const e = min((__float_as_uint(fmaxf(t1, fmaxf(t2, t3))) >> 23) & 0xffu, 253u);
-    float const sc = __uint_as_float((254u - e) << 23);
-    u1 = t1 * sc;
-    u2 = t2 * sc;
-    u3 = t3 * sc;
-  }
-  T const b1 = u2 * u3;
-  T const b2 = T(6.0) * (u1 * u3);
-  T const b3 = T(3.0) * (u1 * u2);
-  return {b1 * r1 + b2 * r2 + b3 * r3, b1 + b2 + b3};
+__device__ __forceinline__ double weno5_q(double d, double eps) {
+  return fma((4.0 / 3.0) * d, d, eps);
+}
+__device__ __forceinline__ Weno5Frac weno5_frac(double g2, double g3, double d1, double d3,
+                                                double q1, double q2, double q3) {
+  double const a = g2 + d1, b = g3 - d3;
+  double const s1 = fma(g2, a, q1), s2 = fma(g2, g3, q2), s3 = fma(g3, b, q3);
+  double const r1 = fma(2.0, a, g2), r2 = fma(2.0, g3, g2), r3 = fma(2.0, g3, b);
+  double const t1 = s1 * s1, t2 = s2 * s2, t3 = s3 * s3;
+  // num = t2 t3 r1 + 3 t1 (2 t3 r2 + t2 r3), den the same with r = 1
+  double const y = 3.0 * t1, z = t3 + t3, p = t2 * t3;
+  return {fma(y, fma(z, r2, t2 * r3), p * r1), fma(y, z + t2, p)};
 }
 
-// v_l + num_l / (6 den_l) and v_r - num_r / (6 den_r). Double: one reciprocal
-// of the product of the two denominators (each between ~1e-22 and ~1e7 |g|^8,
-// so the product stays in range for differences up to ~1e17). Float: one
-// reciprocal per side (a scaled denominator can be as small as the ratio of two
-// smoothness terms, so the product of two could underflow).
-template <typename T>
-__device__ __forceinline__ void weno5_finish(T v_l, Weno5Frac<T> const &l, T v_r,
-                                             Weno5Frac<T> const &r, T &left, T &right) {
-  if constexpr (sizeof(T) == 8) {
-    T const rr = inv((T(6.0) * l.den) * r.den);
-    left = v_l + l.num * (r.den * rr);
-    right = v_r - r.num * (l.den * rr);
-  } else {
-    left = v_l + l.num * inv(T(6.0) * l.den);
-    right = v_r - r.num * inv(T(6.0) * r.den);
-  }
+// num_l / (6 den_l) and num_r / (6 den_r) with one reciprocal: the denominators
+// lie between ~1e-23 (eps^4) and ~1e2 |g|^8, so their product stays in range
+// for differences up to ~1e17.
+__device__ __forceinline__ void weno5_finish(Weno5Frac const &l, Weno5Frac const &r,
+                                             double &left, double &right) {
+  double const rr = inv((6.0 * l.den) * r.den);
+  left = l.num * (r.den * rr);
+  right = r.num * (l.den * rr);
+}
+
+// Both reconstructions of a face from the five first differences of its six
+// cells: the UpwindLeft value is (left cell) + left, the UpwindRight value
+// (right cell) - right. eps is the reference's 1e-6, times the square of the
+// factor by which the caller scaled the differences (WENO5 of scaled data with
+// eps scaled alike is the scaled WENO5).
+__device__ __forceinline__ void weno5_increments(double const (&G)[5], double eps, double &left,
+                                                 double &right) {
+  double const D1 = G[1] - G[0], D2 = G[2] - G[1], D3 = G[3] - G[2], D4 = G[4] - G[3];
+  double const q2 = weno5_q(D2, eps), q3 = weno5_q(D3, eps);
+  weno5_finish(weno5_frac(G[1], G[2], D1, D3, weno5_q(D1, eps), q2, q3),
+               weno5_frac(G[3], G[2], -D4, -D2, weno5_q(D4, eps), q3, q2), left, right);
+}
+// The same for two arrays (flux splitting): UpwindLeft from the differences
+// A[0..3], UpwindRight from B[1..4].
+__device__ __forceinline__ void weno5_increments_two(double const (&A)[5], double const (&B)[5],
+                                                     double eps, double &left, double &right) {
+  double const A1 = A[1] - A[0], A2 = A[2] - A[1], A3 = A[3] - A[2];
+  double const B2 = B[2] - B[1], B3 = B[3] - B[2], B4 = B[4] - B[3];
+  weno5_finish(weno5_frac(A[1], A[2], A1, A3, weno5_q(A1, eps), weno5_q(A2, eps), weno5_q(A3, eps)),
+               weno5_frac(B[3], B[2], -B4, -B2, weno5_q(B4, eps), weno5_q(B3, eps), weno5_q(B2, eps)),
+               left, right);
 }
 
 // ---- packed FP32 pairs (Blackwell f32x2: one instruction for two lanes) ----
@@ -322,9 +317,14 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b
 
 // UpwindLeft and UpwindRight of one face, packed: P_k = (a[k], a[5-k]) for
 // k = 0 .. 4 of the six cells a[0..5] (i-2 .. i+3). Lane y runs the mirrored
-// stencil, whose first differences are the negated ones weno5_frac takes for
-// the right side, so both lanes end as P_2 + num / (6 den) (weno5_frac; the
-// second differences and the e_k enter squared, so their signs do not matter).
+// stencil; both lanes end as P_2 + num / (6 den), with the indicators
+// 13/3 d_k^2 + e_k^2 (four times the reference's, eps likewise) and the ideal
+// weights as 1, 6, 3. The t_k are first multiplied by the power of two that
+// brings the largest into [1, 2) (exact: the scale is built from the exponent
+// bits), so the products stay inside the float range; a product that underflows
+// belongs to a weight below 2^-126 of the largest. One reciprocal per side (a
+// scaled denominator can be as small as the ratio of two smoothness terms, so
+// the product of two could underflow).
 __device__ __forceinline__ float2 weno5_packed(float2 P0, float2 P1, float2 P2, float2 P3,
                                                float2 P4) {
   float2 const ng1 = sub2(P0, P1), g2 = sub2(P2, P1), g3 = sub2(P3, P2), ng4 = sub2(P3, P4);
@@ -354,9 +354,8 @@ __device__ __forceinline__ float2 weno5_packed(float2 P0, float2 P1, float2 P2, 
 }
 
 // UpwindLeft and UpwindRight of one face from the same six cells a[0..5]
-// (i-2..i+3). The fast build shares the first differences and the second
-// differences centred on a[2] and a[3] between the two (double), or runs the
-// two sides as the lanes of packed f32x2 arithmetic (float).
+// (i-2..i+3): weno5_increments (fast build, double) or the two sides as the
+// lanes of packed f32x2 arithmetic (float).
 template <typename T>
 __device__ __forceinline__ void weno5_pair(T const (&a)[6], T &left, T &right) {
   if constexpr (!ALP_FAST) {
@@ -369,11 +368,11 @@ __device__ __forceinline__ void weno5_pair(T const (&a)[6], T &left, T &right) {
     left = r.x;
     right = r.y;
   } else {
-    T const G0 = a[1] - a[0], G1 = a[2] - a[1], G2 = a[3] - a[2], G3 = a[4] - a[3];
-    T const G4 = a[5] - a[4];
-    T const D1 = G1 - G0, D2 = G2 - G1, D3 = G3 - G2, D4 = G4 - G3;
-    weno5_finish(a[2], weno5_frac(G0, G1, G2, G3, D1, D2, D3), a[3],
-                 weno5_frac(G4, G3, G2, G1, D4, D3, D2), left, right);
+    double const G[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], a[5] - a[4]};
+    double l, r;
+    weno5_increments(G, 1.0e-6, l, r);
+    left = a[2] + l;
+    right = a[3] - r;
   }
 }
 
@@ -392,10 +391,12 @@ __device__ __forceinline__ void weno5_two(T const (&a)[6], T const (&b)[6], T &l
     left = r.x;
     right = r.y;
   } else {
-    T const A0 = a[1] - a[0], A1 = a[2] - a[1], A2 = a[3] - a[2], A3 = a[4] - a[3];
-    T const B1 = b[2] - b[1], B2 = b[3] - b[2], B3 = b[4] - b[3], B4 = b[5] - b[4];
-    weno5_finish(a[2], weno5_frac(A0, A1, A2, A3, A1 - A0, A2 - A1, A3 - A2), b[3],
-                 weno5_frac(B4, B3, B2, B1, B4 - B3, B3 - B2, B2 - B1), left, right);
+    double const A[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], 0.0};
+    double const B[5] = {0.0, b[2] - b[1], b[3] - b[2], b[4] - b[3], b[5] - b[4]};
+    double l, r;
+    weno5_increments_two(A, B, 1.0e-6, l, r);
+    left = a[2] + l;
+    right = b[3] - r;
   }
 }
 
@@ -624,7 +625,212 @@ __device__ __forceinline__ void to_physical_packed(Roe<float> const &r, float2 c
   out[ENERGY] = s;
 }
 
+// ---- the fast build's FP64 characteristic frame ------------------------------
+// The same Roe eigensystem with its rows factored. For a difference x =
+// (rho, E, m) of conserved states (or of physical fluxes) let
+//   Dp = mp - up rho, D1 = m1 - u1 rho, D2 = m2 - u2 rho,
+//   V  = (E - H rho - up Dp - u1 D1 - u2 D2) / c^2;
+// the characteristic values of the eigenvector matrices above are then
+//   (u - c, u + c):  ((rho + gru V) -/+ Dp / c) / 2,  entropy wave: -V,
+//   minor waves:     -D1 / rho_roe, D2 / rho_roe.
+// 12 operations per difference against 19 with the rows multiplied out. The
+// constant factors (1/2, 1/rho_roe) are left out of the values and go into the
+// eps of their reconstruction instead (weno5_increments).
+template <int DIM> struct CharFrame {
+  double up, u1, u2, H, gru;       // Roe averages, gamma - 1
+  double c, one_c, cc, one_cc;     // speed of sound, its inverse and squares
+  double Hcc, wp, w1, w2;          // H / c^2, u / c^2
+  double rho2;                     // Roe density squared (the product of the densities)
+};
+
+// Cell quantities of the frame: 1/rho, velocities, pressure, enthalpy, c^2.
+template <int DIM> struct CharCell {
+  double one, up, u1, u2, p, H, cc;
+};
+
+template <int DIM, int DIR>
+__device__ __forceinline__ CharCell<DIM> char_cell(Eos const &e, double const (&c)[DIM + 2]) {
+  constexpr int mP = MOMX + DIR;
+  constexpr int m1 = MOMX + (DIM > 1 ? Minor<DIR>::m1 : 0);
+  constexpr int m2 = MOMX + (DIM > 2 ? Minor<DIR>::m2 : 0);
+  CharCell<DIM> r;
+  r.one = inv(c[MASS]);
+  r.up = c[mP] * r.one;
+  double um = r.up * c[mP];
+  r.u1 = r.u2 = 0.0;
+  if constexpr (DIM > 1) {
+    r.u1 = c[m1] * r.one;
+    um = fma(r.u1, c[m1], um);
+  }
+  if constexpr (DIM > 2) {
+    r.u2 = c[m2] * r.one;
+    um = fma(r.u2, c[m2], um);
+  }
+  double const gB = e.gamma * e.B;
+  double oneH = r.one;
+  if (e.safe && !(c[MASS] > DBL_EPSILON)) {
+    // StiffenedGasSafe divides by max(rho, eps)
+    oneH = 1.0 / DBL_EPSILON;
+    um *= c[MASS] * oneH;
+  }
+  r.p = fma(e.gamma - 1.0, fma(-0.5, um, c[ENERGY]), -gB);
+  if (e.safe) r.p = dmax(r.p, -e.B + DBL_EPSILON);
+  r.H = (c[ENERGY] + r.p) * oneH;
+  r.cc = fma(e.gamma, r.p, gB) * r.one;
+  return r;
+}
+
+// Roe average of the cells t (left) and n: with the weights w_t = 1 / (1 +
+// lambda), lambda = sqrt(rho_n / rho_t), and w_n = lambda w_t, an average is
+// a_n + w_t (a_t - a_n), and c^2 = avg(c^2) + (gamma - 1) w_t w_n |du|^2 / 2
+// (psi + gru p / rho of eigendecomposition.h:262-300 is a cell's own c^2).
+template <int DIM, int DIR>
+__device__ __forceinline__ CharFrame<DIM> char_frame(Eos const &e, CharCell<DIM> const &t,
+                                                     CharCell<DIM> const &n, double rho_t,
+                                                     double rho_n) {
+  CharFrame<DIM> r;
+  double const ratio = rho_n * t.one;
+  double const lambda = ratio * rsqrt_nr(ratio);
+  double const wt = inv(1.0 + lambda);
+  double const du = t.up - n.up;
+  r.up = fma(wt, du, n.up);
+  double d2 = du * du;
+  r.u1 = r.u2 = 0.0;
+  if constexpr (DIM > 1) {
+    double const d = t.u1 - n.u1;
+    r.u1 = fma(wt, d, n.u1);
+    d2 = fma(d, d, d2);
+  }
+  if constexpr (DIM > 2) {
+    double const d = t.u2 - n.u2;
+    r.u2 = fma(wt, d, n.u2);
+    d2 = fma(d, d, d2);
+  }
+  r.H = fma(wt, t.H - n.H, n.H);
+  r.gru = e.gamma - 1.0;
+  r.cc = fma((0.5 * r.gru) * (lambda * (wt * wt)), d2, fma(wt, t.cc - n.cc, n.cc));
+  r.one_c = rsqrt_nr(r.cc);
+  r.c = r.cc * r.one_c;
+  r.one_cc = r.one_c * r.one_c;
+  r.Hcc = r.H * r.one_cc;
+  r.wp = r.up * r.one_cc;
+  r.w1 = r.u1 * r.one_cc;
+  r.w2 = r.u2 * r.one_cc;
+  r.rho2 = rho_t * rho_n;
+  return r;
+}
+
+// Scaled characteristic values of a difference x (conserved-field order) in
+// wave order: 2 (u - c), minor waves -rho_roe / +rho_roe, -entropy, 2 (u + c).
+template <int DIM, int DIR>
+__device__ __forceinline__ void char_project(CharFrame<DIM> const &r, double const (&x)[DIM + 2],
+                                             double (&ch)[DIM + 2]) {
+  constexpr int mP = MOMX + DIR;
+  constexpr int m1 = MOMX + (DIM > 1 ? Minor<DIR>::m1 : 0);
+  constexpr int m2 = MOMX + (DIM > 2 ? Minor<DIR>::m2 : 0);
+  double const rho = x[MASS];
+  double const Dp = fma(-r.up, rho, x[mP]);
+  double V = fma(-r.wp, Dp, fma(-r.Hcc, rho, r.one_cc * x[ENERGY]));
+  if constexpr (DIM > 1) {
+    ch[1] = fma(-r.u1, rho, x[m1]);
+    V = fma(-r.w1, ch[1], V);
+  }
+  if constexpr (DIM > 2) {
+    ch[2] = fma(-r.u2, rho, x[m2]);
+    V = fma(-r.w2, ch[2], V);
+  }
+  double const s = fma(r.gru, V, rho);
+  ch[DIM] = V;
+  ch[0] = fma(-r.one_c, Dp, s);
+  ch[DIM + 1] = fma(r.one_c, Dp, s);
+}
+
+// eps of the reconstruction of wave n in these scales.
+template <int DIM>
+__device__ __forceinline__ double char_eps(CharFrame<DIM> const &r, int n) {
+  return n == 0 || n == DIM + 1 ? 4.0e-6 : (n == DIM ? 1.0e-6 : 1.0e-6 * r.rho2);
+}
+
+// base + sgn (the conserved difference whose scaled characteristic values are ch).
+template <int DIM, int DIR>
+__device__ __forceinline__ void char_restore(CharFrame<DIM> const &r, double const (&base)[DIM + 2],
+                                             double const (&ch)[DIM + 2], double sgn,
+                                             double (&out)[DIM + 2]) {
+  constexpr int mP = MOMX + DIR;
+  constexpr int m1 = MOMX + (DIM > 1 ? Minor<DIR>::m1 : 0);
+  constexpr int m2 = MOMX + (DIM > 2 ? Minor<DIR>::m2 : 0);
+  double const h = 0.5 * sgn;
+  double const rho = fma(h, ch[0] + ch[DIM + 1], (-sgn * r.gru) * ch[DIM]);
+  double const cd = (h * r.c) * (ch[DIM + 1] - ch[0]);
+  out[MASS] = base[MASS] + rho;
+  out[mP] = fma(r.up, rho, base[mP] + cd);
+  double E = fma(r.H, rho, fma(r.up, cd, fma(sgn * r.cc, ch[DIM], base[ENERGY])));
+  if constexpr (DIM > 1) {
+    double const d = sgn * ch[1];
+    out[m1] = fma(r.u1, rho, base[m1] + d);
+    E = fma(r.u1, d, E);
+  }
+  if constexpr (DIM > 2) {
+    double const d = sgn * ch[2];
+    out[m2] = fma(r.u2, rho, base[m2] + d);
+    E = fma(r.u2, d, E);
+  }
+  out[ENERGY] = E;
+}
+
 // ---- HLLC with Einfeldt signal speeds -------------------------------------
+// The fast build's FP64 HLLC: the upwind star flux alone. Where the reference
+// averages the two (S* = 0) they are equal up to rounding: F*_L - F*_R =
+// S* (U*_L - U*_R). With S the unclamped speed of the upwind side, Sc the
+// clamped one, chi = (S - v) / (S - S*) and k = v + Sc (chi - 1), the fluxes are
+//   mass rho k, momentum p + rho (v^2 + Sc (chi S* - v)), minor momenta q k,
+//   energy E k + v p + Sc chi (S* - v) (rho S* + p / (Sc - v)).
+struct HllcUpwind {
+  bool right;        // the upwind side is the right one
+  double rho, p, k;  // its density and pressure; the advecting speed
+  double g, pe;      // momentum per density beside p; energy beside E k
+};
+
+// c^2 of a state (generic_stiffened_gas.h; the safe variant's floors)
+__device__ __forceinline__ double eos_cc(Eos const &e, double rho, double p, double one_rho) {
+  double const gp = e.gamma * (p + e.B);
+  if (e.safe)
+    return dmax(gp * (rho > DBL_EPSILON ? one_rho : inv(dmax(rho, DBL_EPSILON))), DBL_EPSILON);
+  return gp * one_rho;
+}
+
+__device__ __forceinline__ HllcUpwind hllc_upwind(Eos const &e, double rl, double rr, double pl,
+                                                  double pr, double vl, double vr, double one_l,
+                                                  double one_r) {
+  double const ccl = eos_cc(e, rl, pl, one_l), ccr = eos_cc(e, rr, pr, one_r);
+  // Einfeldt: Roe weights wl = 1 / (1 + lambda), wr = lambda wl, lambda = sqrt(rr / rl)
+  double const ratio = rr * one_l;
+  double const lambda = ratio * rsqrt_nr(ratio);
+  double const wl = inv(1.0 + lambda);
+  double const dv = vl - vr;
+  double const u = fma(wl, dv, vr);
+  double const ce2 = fma((0.5 * lambda) * (wl * wl), dv * dv, fma(wl, ccl - ccr, ccr));
+  double const ce = ce2 * rsqrt_nr(ce2);
+  double const cl = ccl * rsqrt_nr(ccl), cr = ccr * rsqrt_nr(ccr);
+  double const sl = dmin(u - ce, vl - cl), sr = dmax(u + ce, vr + cr);
+  double const al = rl * (sl - vl), ar = rr * (sr - vr);
+  double const ss = fma(vl, al, fma(-vr, ar, pr - pl)) * inv(al - ar);
+  HllcUpwind h;
+  h.right = ss < 0.0;
+  h.rho = h.right ? rr : rl;
+  h.p = h.right ? pr : pl;
+  double const v = h.right ? vr : vl;
+  double const s = h.right ? sr : sl;
+  double const sc = h.right ? dmax(sr, 0.0) : dmin(sl, 0.0);
+  double const dss = ss - v;
+  double const dchi = dss * inv(s - ss);  // chi - 1
+  h.k = fma(sc, dchi, v);
+  double const chi = 1.0 + dchi;
+  h.g = fma(v, v, sc * fma(dchi, ss, dss));
+  h.pe = fma(v, h.p, (sc * (chi * dss)) * fma(h.rho, ss, h.p * inv(sc - v)));
+  return h;
+}
+
 // CalculateSignalSpeed, Einfeldt (hll_signal_speed_calculator.h:77-101) and
 // HllcRiemannSolver::SolveRiemannProblemImplementation (hllc_riemann_solver.h:52-198)
 // one_rl, one_rr: 1/density of the two states as returned by inv()
@@ -634,21 +840,24 @@ __device__ __forceinline__ void hllc(Eos const &e, T const (&cl)[DIM + 2], T con
                                      T (&flux)[DIM + 2]) {
   constexpr int NE = DIM + 2;
   constexpr int mP = MOMX + DIR;
+  if constexpr (ALP_FAST && sizeof(T) == 8) {
+    HllcUpwind const h = hllc_upwind(e, cl[MASS], cr[MASS], pres_l, pres_r, vel_l, vel_r, one_rl,
+                                     one_rr);
+    flux[MASS] = h.rho * h.k;
+    flux[mP] = fma(h.rho, h.g, h.p);
+    flux[ENERGY] = fma(h.right ? cr[ENERGY] : cl[ENERGY], h.k, h.pe);
+#pragma unroll
+    for (int d = 0; d < DIM - 1; ++d) {
+      int const mm = MOMX + (d == 0 ? Minor<DIR>::m1 : Minor<DIR>::m2);
+      flux[mm] = (h.right ? cr[mm] : cl[mm]) * h.k;
+    }
+    return;
+  }
   T const c_l = eos_speed_of_sound<T>(e, cl[MASS], pres_l, one_rl);
   T const c_r = eos_speed_of_sound<T>(e, cr[MASS], pres_r, one_rr);
-  T srl, srr, rho_div;
-  if constexpr (ALP_FAST && sizeof(T) == 8) {
-    // the Roe weights themselves (rho_div = 1): lambda = sqrt(rho_r / rho_l),
-    // w_l = 1 / (1 + lambda), w_r = lambda w_l
-    T const lambda = tsqrt(cr[MASS] * one_rl);
-    srl = inv(T(1) + lambda);
-    srr = lambda * srl;
-    rho_div = T(1);
-  } else {
-    srl = tsqrt(cl[MASS]);
-    srr = tsqrt(cr[MASS]);
-    rho_div = quot(T(1), srl + srr);
-  }
+  T const srl = tsqrt(cl[MASS]);
+  T const srr = tsqrt(cr[MASS]);
+  T const rho_div = quot(T(1), srl + srr);
   T const u_roe = ((vel_l * srl) + (vel_r * srr)) * rho_div;
   T const c_e = tsqrt(((c_l * c_l * srl) + (c_r * c_r * srr)) * rho_div +
                      (T(0.5) * srl * srr * rho_div * rho_div) * (vel_r - vel_l) * (vel_r - vel_l));
@@ -656,32 +865,6 @@ __device__ __forceinline__ void hllc(Eos const &e, T const (&cl)[DIM + 2], T con
   T const srs = dmax(u_roe + c_e, vel_r + c_r);
   T const s_star = quot((pres_r - pres_l) + (cl[mP] * (sls - vel_l) - cr[mP] * (srs - vel_r)),
                         cl[MASS] * (sls - vel_l) - cr[MASS] * (srs - vel_r));
-  if constexpr (ALP_FAST) {
-    // The upwind star flux alone. Where the reference averages the two (S* = 0)
-    // they are equal up to rounding: F*_L - F*_R = S* (U*_L - U*_R).
-    bool const rs = s_star < T(0);
-    T const rho = rs ? cr[MASS] : cl[MASS];
-    T const mp = rs ? cr[mP] : cl[mP];
-    T const E = rs ? cr[ENERGY] : cl[ENERGY];
-    T const p = rs ? pres_r : pres_l;
-    T const v = rs ? vel_r : vel_l;
-    T const one_r = rs ? one_rr : one_rl;
-    T const s = rs ? srs : sls;
-    T const sc = rs ? dmax(srs, T(0)) : dmin(sls, T(0));
-    T const chi = quot(s - v, s - s_star);
-    T const rchi = rho * chi;
-    flux[MASS] = mp + (sc * (rchi - rho));
-    flux[mP] = ((mp * mp) * one_r + p) + (sc * (rchi * s_star - mp));
-    T const es = rchi * (E * one_r + (s_star - v) * (s_star + quot(p, rho * (sc - v))));
-    flux[ENERGY] = v * (E + p) + (sc * (es - E));
-#pragma unroll
-    for (int d = 0; d < DIM - 1; ++d) {
-      int const mm = MOMX + (d == 0 ? Minor<DIR>::m1 : Minor<DIR>::m2);
-      T const q = rs ? cr[mm] : cl[mm];
-      flux[mm] = v * q + (sc * (chi * q - q));
-    }
-    return;
-  }
   T const sl = dmin(sls, T(0));
   T const sr = dmax(srs, T(0));
   T const chi_l = quot(sls - vel_l, sls - s_star);

@@ -294,6 +294,7 @@ __device__ __forceinline__ void riemann_ext(int solver, int speeds, Eos const &e
 // Scheme policies of face_compute. The default one is the compiled hot path;
 // ExtPolicy dispatches on SchemeOptions at run time (FP64 only).
 struct DefaultPolicy {
+  static constexpr bool is_default = true;
   template <typename T> __device__ __forceinline__ T left(T const (&a)[6]) const {
     return weno5_left(a);
   }
@@ -327,6 +328,7 @@ struct DefaultPolicy {
 };
 
 struct ExtPolicy {
+  static constexpr bool is_default = false;
   SchemeOptions o;
   double glf[3] = {0.0, 0.0, 0.0};  // GlobalLaxFriedrichs wave speeds of the block's case
   template <int N> __device__ __forceinline__ double left(double const (&a)[N]) const {
