@@ -147,6 +147,10 @@ struct alp_engine {
         ALP_CUDA(alp::launch_pencil_stage(Ls, U, out[s], R, nbr26, cases, s));
       } else if (path == 2) {
         if (int rc = record_overlapped_stage(Ls, out[s], s0 + s)) return rc;
+      } else if (alp::sweep_pays(dim, nwork)) {
+        // the last direction's faces run in the launch that applies the stage
+        ALP_CUDA(launch_face_flux_all(Ls, nbr26, cases, F, stride(), dstride(), face_threads, dim - 1));
+        ALP_CUDA(alp::launch_sweep_update(Ls, U, out[s], F, stride(), dstride(), nbr26, cases, s0 + s));
       } else {
         ALP_CUDA(launch_face_flux_all(Ls, nbr26, cases, F, stride(), dstride(), face_threads));
         ALP_CUDA(launch_stage_update(Ls, U, out[s], F, stride(), dstride(), s0 + s, cases, 0.0));

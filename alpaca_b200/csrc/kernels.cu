@@ -8,410 +8,11 @@
 #include <cstdio>
 
 
-#include "kernels.cuh"
-#include "face.cuh"
-#include "rotate.cuh"
-#include "step_common.cuh"
+#include "face_kernels.cuh"
 
 namespace alp {
 
 namespace {
-
-__device__ __forceinline__ int slot_of(int const *work, int item) {
-  return work ? work[item] : item;
-}
-
-// ---------------------------------------------------------------------------
-// face flux
-// ---------------------------------------------------------------------------
-
-template <int DIM, int DIR> struct FaceMap {
-  static constexpr int O1 = DIR == 0 ? 1 : 0;
-  static constexpr int O2 = DIR == 2 ? 1 : 2;
-  static constexpr int E1 = Geo<DIM>::ic(O1);
-  static constexpr int E2 = Geo<DIM>::ic(O2);
-  static constexpr int COUNT = (IC + 1) * E1 * E2;
-  // Thread t -> face (a along DIR, p1, p2 across). Consecutive threads walk the
-  // fastest-varying stored dimension so that stencil loads coalesce.
-  __device__ static void decode(int t, int &a, int &p1, int &p2) {
-    if constexpr (DIR == DIM - 1) {
-      a = t % (IC + 1);
-      int const r = t / (IC + 1);
-      p1 = r / E2;
-      p2 = r % E2;
-    } else {
-      a = t / (E1 * E2);
-      p1 = (t / E2) % E1;
-      p2 = t % E2;
-    }
-  }
-};
-
-// Minimum resident 128-thread CTAs per SM of the face kernels, which caps
-// their registers (168 / 128 / 102 at 3 / 4 / 5); compile-time tunable.
-// Measured on the FP64 128^3 step: FV char 4 CTAs 1.60 ms vs 3: 1.71, 5: 1.66;
-// FV prim 5: 1.37 vs 4: 1.46, 6: 1.37; flux splitting 3: 1.91 vs 1-2: 2.23
-// (at 4 it spills ~0.7 KB per thread).
-#ifndef ALP_FS_ROE_CTAS
-#define ALP_FS_ROE_CTAS 3
-#endif
-#ifndef ALP_FV_CHAR_CTAS
-#define ALP_FV_CHAR_CTAS 4
-#endif
-#ifndef ALP_FV_PRIM_CTAS
-#define ALP_FV_PRIM_CTAS 5
-#endif
-// FP32-flux instantiations (fewer live doubles) have their own limits
-// (measured on the 128^3 step: FS 4 CTAs 2.05 ms vs 3: 2.23, 2: 2.86; FV
-// char 5 CTAs 1.56 ms vs 4: 1.64, 6: 1.59; FV prim 5: 1.455 vs 6: 1.48).
-#ifndef ALP_FS_ROE_CTAS_F32
-#define ALP_FS_ROE_CTAS_F32 4
-#endif
-#ifndef ALP_FV_CHAR_CTAS_F32
-#define ALP_FV_CHAR_CTAS_F32 5
-#endif
-#ifndef ALP_FV_PRIM_CTAS_F32
-#define ALP_FV_PRIM_CTAS_F32 ALP_FV_PRIM_CTAS
-#endif
-template <int SCHEME, typename T = double> struct FaceOccupancy {
-  static constexpr bool f32 = sizeof(T) == 4;
-  static constexpr int min_ctas =
-      SCHEME == FV_CHAR ? (f32 ? ALP_FV_CHAR_CTAS_F32 : ALP_FV_CHAR_CTAS)
-      : SCHEME == FV_PRIM ? (f32 ? ALP_FV_PRIM_CTAS_F32 : ALP_FV_PRIM_CTAS)
-                          : (f32 ? ALP_FS_ROE_CTAS_F32 : ALP_FS_ROE_CTAS);
-};
-
-// Stores one face's fluxes in the reference flux-array layout: = (zero for a
-// skipped face) or, for the drop-in contract, += (skipped faces untouched).
-template <int DIM, int DIR, bool ACCUM>
-__device__ __forceinline__ void write_flux(double *__restrict__ F, int item, long long stride,
-                                           int a, int p1, int p2, bool valid,
-                                           double const (&flux)[DIM + 2]) {
-  using G = Geo<DIM>;
-  using M = FaceMap<DIM, DIR>;
-  int fi[3];
-  fi[DIR] = a;
-  fi[M::O1] = p1 + 1;
-  fi[M::O2] = p2 + 1;
-  double *fo = F + (long long)item * stride + G::face(fi[0], fi[1], fi[2]);
-#pragma unroll
-  for (int f = 0; f < DIM + 2; ++f) {
-    double const v = valid ? flux[f] : 0.0;
-    if (ACCUM) {
-      if (valid) fo[f * G::FACES] += v;
-    } else {
-      fo[f * G::FACES] = v;
-    }
-  }
-}
-
-// Stencil of the face a (between cells a-1 and a along DIR) at transverse
-// position (p1, p2): cells a-3 .. a+2 in interior numbering, all fields.
-// GATHER: cells outside the interior along DIR come from the neighbour blocks'
-// interiors (nbr26; zero gradient at domain faces) instead of the block's own
-// halo cells, so no halo copy is needed between stages.
-template <int DIM, int DIR, bool GATHER>
-__device__ __forceinline__ double const *stencil_cell(double const *__restrict__ U,
-                                                      double const *blk, int c, int cell0,
-                                                      int nlo, int nhi) {
-  using G = Geo<DIM>;
-  constexpr int step = DIR == 0 ? G::TCY * G::TCZ : (DIR == 1 ? G::TCZ : 1);
-  // cell0: offset of (transverse position, DIR index 0) in the block
-  if (GATHER && c < HS)
-    return nlo >= 0 ? U + (size_t)nlo * G::BLOCK_DOUBLES + cell0 + (c + IC) * step
-                    : blk + cell0 + HS * step;
-  if (GATHER && c >= HS + IC)
-    return nhi >= 0 ? U + (size_t)nhi * G::BLOCK_DOUBLES + cell0 + (c - IC) * step
-                    : blk + cell0 + (HS + IC - 1) * step;
-  return blk + cell0 + c * step;
-}
-
-template <int DIM, int DIR>
-__device__ __forceinline__ int line_origin(int p1, int p2) {
-  using G = Geo<DIM>;
-  using M = FaceMap<DIM, DIR>;
-  int c[3];
-  c[DIR] = 0;
-  c[M::O1] = G::fic(M::O1) + p1;
-  c[M::O2] = G::fic(M::O2) + p2;
-  return G::cell(c[0], c[1], c[2]);
-}
-
-template <int DIM, int DIR>
-__device__ __forceinline__ void load_cell(double const *src, double (&dst)[DIM + 2]) {
-#pragma unroll
-  for (int f = 0; f < DIM + 2; ++f) dst[f] = __ldg(src + f * Geo<DIM>::CELLS);
-}
-
-// Cell c of a stencil line (stencil_cell), with symmetry walls: a neighbour
-// entry of -2 across the block face mirrors the line about the wall and negates
-// the momentum normal to it (symmetry_boundary_condition.h:60-113, 148-217;
-// boundary_constants.h:35-46, 167-209); -1 is zero gradient.
-template <int DIM, int DIR, bool GATHER>
-__device__ __forceinline__ void stencil_load(double const *__restrict__ U, double const *blk,
-                                             int c, int cell0, int nlo, int nhi,
-                                             double (&dst)[DIM + 2]) {
-  constexpr int step = DIR == 0 ? Geo<DIM>::TCY * Geo<DIM>::TCZ : (DIR == 1 ? Geo<DIM>::TCZ : 1);
-  if (GATHER && ((c < HS && nlo == -2) || (c >= HS + IC && nhi == -2))) {
-    int const m = c < HS ? 2 * HS - 1 - c : 2 * (HS + IC) - 1 - c;
-    load_cell<DIM, DIR>(blk + cell0 + m * step, dst);
-    dst[MOMX + DIR] = -1.0 * dst[MOMX + DIR];
-    return;
-  }
-  load_cell<DIM, DIR>(stencil_cell<DIM, DIR, GATHER>(U, blk, c, cell0, nlo, nhi), dst);
-}
-
-// Flux of the face with thread index t of direction DIR of the block in `slot`.
-template <int DIM, int DIR, int SCHEME, typename T, bool ACCUM, bool GATHER,
-          typename P = DefaultPolicy, int W = 6>
-__device__ __forceinline__ void face_flux(double const *__restrict__ U,
-                                          int const *__restrict__ nbr26, int slot, int item,
-                                          int t, BlockMeta const &bm, double *__restrict__ F,
-                                          long long stride, P const &pol = P()) {
-  using G = Geo<DIM>;
-  using M = FaceMap<DIM, DIR>;
-  constexpr int NE = G::NE;
-  Eos const eos{bm.gamma, bm.B, bm.safe};
-  int a, p1, p2;
-  M::decode(t, a, p1, p2);
-  double const *blk = U + (size_t)slot * G::BLOCK_DOUBLES;
-  int const cell0 = line_origin<DIM, DIR>(p1, p2);
-  // low / high neighbour along DIR (26-table slots of W,E / S,N / B,T)
-  constexpr int lo_slot = DIR == 0 ? 4 : (DIR == 1 ? 10 : 12);
-  constexpr int hi_slot = DIR == 0 ? 21 : (DIR == 1 ? 15 : 13);
-  int const nlo = GATHER && a < W / 2 ? __ldg(nbr26 + (size_t)slot * 26 + lo_slot) : 0;
-  int const nhi = GATHER && a > IC - W / 2 ? __ldg(nbr26 + (size_t)slot * 26 + hi_slot) : 0;
-  double cons[W][NE];
-#pragma unroll
-  for (int m = 0; m < W; ++m)
-    stencil_load<DIM, DIR, GATHER>(U, blk, HS + a - W / 2 + m, cell0, nlo, nhi, cons[m]);
-  double fd[NE];
-  bool valid;
-  if constexpr (DIM == 3 && DIR != 0) {
-    // 3D y and z faces: the x-face computation of the rotated stencil
-    // (canon_field), the same code as the fused tile kernel
-    double rc[W][NE];
-#pragma unroll
-    for (int m = 0; m < W; ++m)
-#pragma unroll
-      for (int c = 0; c < NE; ++c) rc[m][c] = cons[m][canon_field(DIR, c)];
-    double rf[NE];
-    valid = face_compute<3, 0, SCHEME, T, P, W>(eos, bm.B, rc, rf, pol);
-#pragma unroll
-    for (int c = 0; c < NE; ++c) fd[canon_field(DIR, c)] = rf[c];
-  } else {
-    valid = face_compute<DIM, DIR, SCHEME, T, P, W>(eos, bm.B, cons, fd, pol);
-  }
-  write_flux<DIM, DIR, ACCUM>(F, item, stride, a, p1, p2, valid, fd);
-}
-
-// One direction over all work items (drop-in calls: halos from the buffer).
-template <int DIM, int DIR, int SCHEME, typename T, bool ACCUM>
-__global__ void __launch_bounds__(128, FaceOccupancy<SCHEME, T>::min_ctas)
-face_flux_kernel(double const *__restrict__ U, int const *__restrict__ work,
-                 BlockMeta const *__restrict__ meta, BlockMeta def, double *__restrict__ F,
-                 long long stride) {
-  int const t = blockIdx.y * blockDim.x + threadIdx.x;
-  if (t >= FaceMap<DIM, DIR>::COUNT) return;
-  int const item = blockIdx.x;
-  int const slot = slot_of(work, item);
-  BlockMeta const bm = meta ? meta[slot] : def;
-  face_flux<DIM, DIR, SCHEME, T, ACCUM, false>(U, nullptr, slot, item, t, bm, F, stride);
-}
-
-// Every direction of every work item in one launch (engine): blockIdx.z is the
-// direction, stencils gathered from neighbours, direction d written to
-// F + d * dstride. Items whose case is inactive (dt == 0) are skipped.
-template <int DIM, int SCHEME, typename T>
-__global__ void __launch_bounds__(128, FaceOccupancy<SCHEME, T>::min_ctas)
-face_flux_all_kernel(double const *__restrict__ U, int const *__restrict__ work,
-                     BlockMeta const *__restrict__ meta, int const *__restrict__ nbr26,
-                     CaseState const *__restrict__ cases, double *__restrict__ F,
-                     long long stride, long long dstride, int chunks,
-                     int const *__restrict__ items) {
-  // grid (items x chunks, 1, dir): an item's chunks are consecutive, so the
-  // CTAs resident at any time share few blocks' stencils (a few MB of L2
-  // instead of one stencil plane of every item in the launch). items (when
-  // given): the work-list position of each launch position
-  int const chunk = (int)(blockIdx.x % chunks);
-  int const pos = (int)(blockIdx.x / chunks);
-  int const item = items ? items[pos] : pos;
-  int const t = chunk * blockDim.x + threadIdx.x;
-  int const slot = work[item];
-  BlockMeta const bm = meta[slot];
-  if (!(cases[bm.case_id].dt > 0.0)) return;
-  int const dir = blockIdx.z;
-  if (dir == 0) {
-    if (t < FaceMap<DIM, 0>::COUNT)
-      face_flux<DIM, 0, SCHEME, T, false, true>(U, nbr26, slot, item, t, bm, F, stride);
-  } else if (DIM > 1 && dir == 1) {
-    if (t < FaceMap<DIM, 1>::COUNT)
-      face_flux<DIM, (DIM > 1 ? 1 : 0), SCHEME, T, false, true>(U, nbr26, slot, item, t, bm,
-                                                                 F + dstride, stride);
-  } else if (DIM > 2) {
-    if (t < FaceMap<DIM, 2>::COUNT)
-      face_flux<DIM, (DIM > 2 ? 2 : 0), SCHEME, T, false, true>(U, nbr26, slot, item, t, bm,
-                                                                 F + 2 * dstride, stride);
-  }
-}
-
-// The run-time selected schemes read 6-cell stencils (i-2 .. i+3), or 8-cell
-// stencils (i-3 .. i+4) when the stencil is WENO7; the narrower stencils use
-// the middle cells. The 8-wide instantiation holds 33 % more stencil state, so
-// the launchers pick it only for WENO7.
-inline bool ext_wide(SchemeOptions const &o) { return o.stencil == ST_WENO7; }
-
-// The policy of one block: the GlobalLaxFriedrichs wave speeds of its case.
-__device__ __forceinline__ ExtPolicy block_policy(ExtPolicy pol, BlockMeta const &bm,
-                                                  unsigned long long const *glf) {
-  if (glf && pol.o.splitting == FSP_GLF)
-    for (int k = 0; k < 3; ++k) pol.glf[k] = __longlong_as_double(glf[4 * bm.case_id + k]);
-  return pol;
-}
-
-// The same two kernels for the run-time selected schemes (ExtPolicy, FP64).
-template <int DIM, int DIR, int SCHEME, bool ACCUM, int W>
-__global__ void __launch_bounds__(128)
-face_flux_ext_kernel(double const *__restrict__ U, int const *__restrict__ work,
-                     BlockMeta const *__restrict__ meta, BlockMeta def, double *__restrict__ F,
-                     long long stride, ExtPolicy pol, unsigned long long const *__restrict__ glf) {
-  int const t = blockIdx.y * blockDim.x + threadIdx.x;
-  if (t >= FaceMap<DIM, DIR>::COUNT) return;
-  int const item = blockIdx.x;
-  int const slot = slot_of(work, item);
-  BlockMeta const bm = meta ? meta[slot] : def;
-  face_flux<DIM, DIR, SCHEME, double, ACCUM, false, ExtPolicy, W>(U, nullptr, slot, item, t, bm, F,
-                                                               stride, block_policy(pol, bm, glf));
-}
-
-template <int DIM, int SCHEME, int W>
-__global__ void __launch_bounds__(128)
-face_flux_all_ext_kernel(double const *__restrict__ U, int const *__restrict__ work,
-                         BlockMeta const *__restrict__ meta, int const *__restrict__ nbr26,
-                         CaseState const *__restrict__ cases, double *__restrict__ F,
-                         long long stride, long long dstride, ExtPolicy pol0,
-                         unsigned long long const *__restrict__ glf,
-                         int const *__restrict__ items) {
-  int const t = blockIdx.y * blockDim.x + threadIdx.x;
-  int const item = items ? items[blockIdx.x] : (int)blockIdx.x;
-  int const slot = work[item];
-  BlockMeta const bm = meta[slot];
-  if (!(cases[bm.case_id].dt > 0.0)) return;
-  ExtPolicy const pol = block_policy(pol0, bm, glf);
-  int const dir = blockIdx.z;
-  if (dir == 0) {
-    if (t < FaceMap<DIM, 0>::COUNT)
-      face_flux<DIM, 0, SCHEME, double, false, true, ExtPolicy, W>(U, nbr26, slot, item, t, bm, F,
-                                                                stride, pol);
-  } else if (DIM > 1 && dir == 1) {
-    if (t < FaceMap<DIM, 1>::COUNT)
-      face_flux<DIM, (DIM > 1 ? 1 : 0), SCHEME, double, false, true, ExtPolicy, W>(
-          U, nbr26, slot, item, t, bm, F + dstride, stride, pol);
-  } else if (DIM > 2) {
-    if (t < FaceMap<DIM, 2>::COUNT)
-      face_flux<DIM, (DIM > 2 ? 2 : 0), SCHEME, double, false, true, ExtPolicy, W>(
-          U, nbr26, slot, item, t, bm, F + 2 * dstride, stride, pol);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// pencil sweeps (engine fast path)
-// ---------------------------------------------------------------------------
-
-// Interior linear index of the cell with index c along DIR at transverse (p1, p2).
-template <int DIM, int DIR>
-__device__ __forceinline__ int interior_index(int c, int p1, int p2) {
-  using M = FaceMap<DIM, DIR>;
-  int ci[3] = {0, 0, 0};
-  ci[DIR] = c;
-  ci[M::O1] = p1;
-  ci[M::O2] = p2;
-  if constexpr (DIM == 3) return (ci[0] * IC + ci[1]) * IC + ci[2];
-  else if constexpr (DIM == 2) return ci[0] * IC + ci[1];
-  else return ci[0];
-}
-
-// One thread walks a line of 16 cells along DIR: it computes the 17 face
-// fluxes in order with a sliding 6-cell stencil window (each cell is loaded
-// once per line instead of six times) and forms each cell's flux difference
-// F(a-1/2) - F(a+1/2) as soon as both faces are known. The directions run one
-// after the other: MODE 0 stores the difference in R, MODE 1 adds to R, MODE 2
-// (the last direction) adds, scales by 1/cell size and applies the SSP-RK3
-// stage: Uout = (stage ? a0 Uin + a1 U0 : Uin) + c dt rhs. The summation order
-// is therefore (dx + dy) + dz instead of the reference's three-order symmetric
-// sum (the strict build keeps that one). Stencils are gathered from neighbour
-// interiors; cases with dt == 0 are skipped.
-template <int DIM, int DIR, int SCHEME, typename T, int MODE>
-__global__ void __launch_bounds__(128, FaceOccupancy<SCHEME>::min_ctas)
-pencil_kernel(double const *Uin, double const *U0, double *Uout, double *R,
-              int const *__restrict__ work, int nwork, BlockMeta const *__restrict__ meta,
-              int const *__restrict__ nbr26, CaseState const *__restrict__ cases, int stage) {
-  using G = Geo<DIM>;
-  using M = FaceMap<DIM, DIR>;
-  constexpr int NE = G::NE;
-  constexpr int P = M::E1 * M::E2;  // lines per block
-  constexpr int step = DIR == 0 ? G::TCY * G::TCZ : (DIR == 1 ? G::TCZ : 1);
-  constexpr int lo_slot = DIR == 0 ? 4 : (DIR == 1 ? 10 : 12);
-  constexpr int hi_slot = DIR == 0 ? 21 : (DIR == 1 ? 15 : 13);
-  int const g = blockIdx.x * blockDim.x + threadIdx.x;
-  int const item = g / P;
-  if (item >= nwork) return;
-  int const p = g - item * P;
-  int const p1 = p / M::E2, p2 = p - (p / M::E2) * M::E2;
-  int const slot = work[item];
-  BlockMeta const bm = meta[slot];
-  double const dt = cases[bm.case_id].dt;
-  if (!(dt > 0.0)) return;
-  Eos const eos{bm.gamma, bm.B, bm.safe};
-  double const *blk = Uin + (size_t)slot * G::BLOCK_DOUBLES;
-  int const cell0 = line_origin<DIM, DIR>(p1, p2);
-  int const nlo = __ldg(nbr26 + (size_t)slot * 26 + lo_slot);
-  int const nhi = __ldg(nbr26 + (size_t)slot * 26 + hi_slot);
-  double *Rb = R ? R + (size_t)slot * NE * G::INTERIOR : nullptr;
-
-  double w[6][NE];
-#pragma unroll
-  for (int m = 0; m < 6; ++m)
-    stencil_load<DIM, DIR, true>(Uin, blk, HS - 3 + m, cell0, nlo, nhi, w[m]);
-  double const ocs = inv(bm.cell_size);
-  RkStage const rk = rk_stage(stage, dt);
-  double fprev[NE];
-#pragma unroll 1
-  for (int a = 0; a <= IC; ++a) {
-    double f[NE];
-    bool const valid = face_compute<DIM, DIR, SCHEME, T>(eos, bm.B, w, f);
-#pragma unroll
-    for (int n = 0; n < NE; ++n)
-      if (!valid) f[n] = 0.0;
-    if (a > 0) {
-      int const ix = interior_index<DIM, DIR>(a - 1, p1, p2);
-      size_t const x = (size_t)slot * G::BLOCK_DOUBLES + cell0 + (HS + a - 1) * step;
-#pragma unroll
-      for (int n = 0; n < NE; ++n) {
-        double const d = fprev[n] - f[n];
-        if constexpr (MODE == 0) {
-          Rb[n * G::INTERIOR + ix] = d;
-        } else if constexpr (MODE == 1) {
-          Rb[n * G::INTERIOR + ix] += d;
-        } else {
-          double const sum = DIM > 1 ? Rb[n * G::INTERIOR + ix] + d : d;
-          double const rhs = 0.0 + sum * ocs;
-          size_t const xf = x + (size_t)n * G::CELLS;
-          Uout[xf] = rk_apply(rk, Uin[xf], rk.first ? 0.0 : U0[xf], rhs);
-        }
-      }
-    }
-#pragma unroll
-    for (int n = 0; n < NE; ++n) fprev[n] = f[n];
-    if (a < IC) {
-#pragma unroll
-      for (int m = 0; m < 5; ++m)
-#pragma unroll
-        for (int n = 0; n < NE; ++n) w[m][n] = w[m + 1][n];
-      stencil_load<DIM, DIR, true>(Uin, blk, HS + a + 3, cell0, nlo, nhi, w[5]);
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------
 // divergence, stage update
@@ -750,91 +351,9 @@ initial_condition_kernel(double *__restrict__ U, int first, int nbx, int nby, in
 
 namespace {
 
-template <int DIM, int DIR, bool ACC, int W>
-cudaError_t face_flux_ext_dir(Launch const &L, dim3 grid, double *F, long long stride,
-                              int threads) {
-  ExtPolicy const pol{L.opt};
-  switch (L.scheme) {
-    case FV_CHAR:
-      face_flux_ext_kernel<DIM, DIR, FV_CHAR, ACC, W>
-          <<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, L.def, F, stride, pol, L.glf);
-      break;
-    case FV_PRIM:
-      face_flux_ext_kernel<DIM, DIR, FV_PRIM, ACC, W>
-          <<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, L.def, F, stride, pol, L.glf);
-      break;
-    case FS_ROE:
-      face_flux_ext_kernel<DIM, DIR, FS_ROE, ACC, W>
-          <<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, L.def, F, stride, pol, L.glf);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-template <int DIM, int DIR, typename T, bool ACC>
-cudaError_t face_flux_dir(Launch const &L, double *F, long long stride, int threads) {
-  using M = FaceMap<DIM, DIR>;
-  dim3 grid(L.nwork, (M::COUNT + threads - 1) / threads);
-  if (!L.opt.is_default())
-    return ext_wide(L.opt) ? face_flux_ext_dir<DIM, DIR, ACC, 8>(L, grid, F, stride, threads)
-                           : face_flux_ext_dir<DIM, DIR, ACC, 6>(L, grid, F, stride, threads);
-  switch (L.scheme) {
-    case FV_CHAR:
-      face_flux_kernel<DIM, DIR, FV_CHAR, T, ACC>
-          <<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, L.def, F, stride);
-      break;
-    case FV_PRIM:
-      face_flux_kernel<DIM, DIR, FV_PRIM, T, ACC>
-          <<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, L.def, F, stride);
-      break;
-    case FS_ROE:
-      face_flux_kernel<DIM, DIR, FS_ROE, T, ACC>
-          <<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, L.def, F, stride);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-template <int DIM, typename T, bool ACC>
-cudaError_t face_flux_dim(Launch const &L, int dir, double *F, long long stride, int threads) {
-  if (dir == 0) return face_flux_dir<DIM, 0, T, ACC>(L, F, stride, threads);
-  if constexpr (DIM > 1)
-    if (dir == 1) return face_flux_dir<DIM, 1, T, ACC>(L, F, stride, threads);
-  if constexpr (DIM > 2)
-    if (dir == 2) return face_flux_dir<DIM, 2, T, ACC>(L, F, stride, threads);
-  return cudaErrorInvalidValue;
-}
-
-template <typename T, bool ACC>
-cudaError_t face_flux_t(Launch const &L, int dir, double *F, long long stride, int threads) {
-  switch (L.dim) {
-    case 1: return face_flux_dim<1, T, ACC>(L, dir, F, stride, threads);
-    case 2: return face_flux_dim<2, T, ACC>(L, dir, F, stride, threads);
-    case 3: return face_flux_dim<3, T, ACC>(L, dir, F, stride, threads);
-  }
-  return cudaErrorInvalidValue;
-}
-
 int interior_of(int dim) { return dim == 3 ? 4096 : (dim == 2 ? 256 : 16); }
 
 }  // namespace
-
-cudaError_t launch_face_flux(Launch const &L, int dir, double *F, long long stride, bool accumulate,
-                             int block_threads) {
-  if (L.nwork <= 0) return cudaSuccess;
-  int const threads = block_threads > 0 ? block_threads : 128;
-  if (threads > 128 || (threads & 31)) return cudaErrorInvalidValue;
-  if (!L.opt.is_default() && L.precision != FP64) return cudaErrorInvalidValue;
-  if (L.precision == FP32_FLUX)
-    return accumulate ? face_flux_t<float, true>(L, dir, F, stride, threads)
-                      : face_flux_t<float, false>(L, dir, F, stride, threads);
-  return accumulate ? face_flux_t<double, true>(L, dir, F, stride, threads)
-                    : face_flux_t<double, false>(L, dir, F, stride, threads);
-}
 
 cudaError_t launch_divergence(Launch const &L, double const *F, long long stride,
                               long long dstride, double *rhs) {
@@ -863,132 +382,6 @@ cudaError_t launch_stage_update(Launch const &L, double const *U0, double *Uout,
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
-}
-
-namespace {
-template <int DIM, int W>
-cudaError_t face_flux_all_ext(Launch const &L, dim3 grid, int const *nbr26, CaseState const *cases,
-                              double *F, long long stride, long long dstride, int threads) {
-  ExtPolicy const pol{L.opt};
-  switch (L.scheme) {
-    case FV_CHAR:
-      face_flux_all_ext_kernel<DIM, FV_CHAR, W><<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, nbr26, cases, F, stride, dstride, pol, L.glf, L.items);
-      break;
-    case FV_PRIM:
-      face_flux_all_ext_kernel<DIM, FV_PRIM, W><<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, nbr26, cases, F, stride, dstride, pol, L.glf, L.items);
-      break;
-    case FS_ROE:
-      face_flux_all_ext_kernel<DIM, FS_ROE, W><<<grid, threads, 0, L.stream>>>(L.U, L.work, L.meta, nbr26, cases, F, stride, dstride, pol, L.glf, L.items);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-template <int DIM, typename T>
-cudaError_t face_flux_all_t(Launch const &L, int const *nbr26, CaseState const *cases, double *F,
-                            long long stride, long long dstride, int threads) {
-  int const count = (IC + 1) * (DIM > 1 ? IC : 1) * (DIM > 2 ? IC : 1);
-  dim3 grid(L.nwork, (count + threads - 1) / threads, DIM);
-  if (!L.opt.is_default())
-    return ext_wide(L.opt)
-               ? face_flux_all_ext<DIM, 8>(L, grid, nbr26, cases, F, stride, dstride, threads)
-               : face_flux_all_ext<DIM, 6>(L, grid, nbr26, cases, F, stride, dstride, threads);
-  // items x chunks < 2^31 for up to 2^31 / 68 items (64-thread chunks)
-  int const chunks = (count + threads - 1) / threads;
-  if ((long long)L.nwork * chunks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  dim3 const g2((unsigned)(L.nwork * chunks), 1, DIM);
-  switch (L.scheme) {
-    case FV_CHAR:
-      face_flux_all_kernel<DIM, FV_CHAR, T><<<g2, threads, 0, L.stream>>>(L.U, L.work, L.meta, nbr26, cases, F, stride, dstride, chunks, L.items);
-      break;
-    case FV_PRIM:
-      face_flux_all_kernel<DIM, FV_PRIM, T><<<g2, threads, 0, L.stream>>>(L.U, L.work, L.meta, nbr26, cases, F, stride, dstride, chunks, L.items);
-      break;
-    case FS_ROE:
-      face_flux_all_kernel<DIM, FS_ROE, T><<<g2, threads, 0, L.stream>>>(L.U, L.work, L.meta, nbr26, cases, F, stride, dstride, chunks, L.items);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-}  // namespace
-
-namespace {
-template <int DIM, int DIR, typename T, int MODE>
-cudaError_t pencil_t(Launch const &L, double const *U0, double *Uout, double *R, int const *nbr26,
-                     CaseState const *cases, int stage) {
-  constexpr int P = FaceMap<DIM, DIR>::E1 * FaceMap<DIM, DIR>::E2;
-  long long const threads = (long long)L.nwork * P;
-  dim3 grid((unsigned)((threads + 127) / 128));
-  switch (L.scheme) {
-    case FV_CHAR:
-      pencil_kernel<DIM, DIR, FV_CHAR, T, MODE><<<grid, 128, 0, L.stream>>>(L.U, U0, Uout, R, L.work, L.nwork, L.meta, nbr26, cases, stage);
-      break;
-    case FV_PRIM:
-      pencil_kernel<DIM, DIR, FV_PRIM, T, MODE><<<grid, 128, 0, L.stream>>>(L.U, U0, Uout, R, L.work, L.nwork, L.meta, nbr26, cases, stage);
-      break;
-    case FS_ROE:
-      pencil_kernel<DIM, DIR, FS_ROE, T, MODE><<<grid, 128, 0, L.stream>>>(L.U, U0, Uout, R, L.work, L.nwork, L.meta, nbr26, cases, stage);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-template <int DIM, typename T>
-cudaError_t pencil_dim(Launch const &L, double const *U0, double *Uout, double *R, int const *nbr26,
-                       CaseState const *cases, int stage) {
-  if (cudaError_t e = pencil_t<DIM, 0, T, DIM == 1 ? 2 : 0>(L, U0, Uout, R, nbr26, cases, stage))
-    return e;
-  if constexpr (DIM > 1)
-    if (cudaError_t e = pencil_t<DIM, (DIM > 1 ? 1 : 0), T, DIM == 2 ? 2 : 1>(L, U0, Uout, R, nbr26, cases, stage))
-      return e;
-  if constexpr (DIM > 2)
-    if (cudaError_t e = pencil_t<DIM, (DIM > 2 ? 2 : 0), T, 2>(L, U0, Uout, R, nbr26, cases, stage))
-      return e;
-  return cudaSuccess;
-}
-}  // namespace
-
-cudaError_t launch_pencil_stage(Launch const &L, double const *U0, double *Uout, double *R,
-                                int const *nbr26, CaseState const *cases, int stage) {
-  if (L.nwork <= 0) return cudaSuccess;
-  if (!L.work || !L.meta || !nbr26 || !cases || stage < 0 || stage > 2) return cudaErrorInvalidValue;
-  if (L.dim > 1 && !R) return cudaErrorInvalidValue;
-  if (!L.opt.is_default()) return cudaErrorInvalidValue;  // pencils: default schemes only
-  bool const f32 = L.precision == FP32_FLUX;
-  switch (L.dim) {
-    case 1: return f32 ? pencil_dim<1, float>(L, U0, Uout, R, nbr26, cases, stage)
-                       : pencil_dim<1, double>(L, U0, Uout, R, nbr26, cases, stage);
-    case 2: return f32 ? pencil_dim<2, float>(L, U0, Uout, R, nbr26, cases, stage)
-                       : pencil_dim<2, double>(L, U0, Uout, R, nbr26, cases, stage);
-    case 3: return f32 ? pencil_dim<3, float>(L, U0, Uout, R, nbr26, cases, stage)
-                       : pencil_dim<3, double>(L, U0, Uout, R, nbr26, cases, stage);
-  }
-  return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_face_flux_all(Launch const &L, int const *nbr26, CaseState const *cases,
-                                 double *F, long long stride, long long dstride, int threads) {
-  if (L.nwork <= 0) return cudaSuccess;
-  if (!L.work || !L.meta || !nbr26 || !cases) return cudaErrorInvalidValue;
-  if (threads <= 0) threads = 128;
-  if (threads > 128 || (threads & 31)) return cudaErrorInvalidValue;
-  if (!L.opt.is_default() && L.precision != FP64) return cudaErrorInvalidValue;
-  bool const f32 = L.precision == FP32_FLUX;
-  switch (L.dim) {
-    case 1: return f32 ? face_flux_all_t<1, float>(L, nbr26, cases, F, stride, dstride, threads)
-                       : face_flux_all_t<1, double>(L, nbr26, cases, F, stride, dstride, threads);
-    case 2: return f32 ? face_flux_all_t<2, float>(L, nbr26, cases, F, stride, dstride, threads)
-                       : face_flux_all_t<2, double>(L, nbr26, cases, F, stride, dstride, threads);
-    case 3: return f32 ? face_flux_all_t<3, float>(L, nbr26, cases, F, stride, dstride, threads)
-                       : face_flux_all_t<3, double>(L, nbr26, cases, F, stride, dstride, threads);
-  }
-  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_rk_stage_rhs(int dim, double *U, double *U0, double const *rhs, int nb,

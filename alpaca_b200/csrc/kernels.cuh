@@ -87,9 +87,20 @@ cudaError_t launch_divergence(Launch const &L, double const *F, long long flux_i
 // stencils gathered from neighbour interiors through nbr26 (zero gradient at
 // domain faces), so block halos are never read; items of inactive cases
 // (dt == 0) skipped. Direction d goes to F + d * dir_stride.
+// dirs: the first `dirs` directions only (0: all).
 cudaError_t launch_face_flux_all(Launch const &L, int const *nbr26, CaseState const *cases,
                                  double *F, long long flux_item_stride, long long dir_stride,
-                                 int threads = 128);
+                                 int threads = 128, int dirs = 0);
+
+// The last direction's faces and the stage update of every work item in one
+// launch (2D, 3D); F holds the other directions' fluxes (launch_face_flux_all
+// with dirs = dim - 1). Same arithmetic, hence the same bits, as
+// launch_face_flux_all of every direction followed by launch_stage_update.
+// sweep_pays: whether nwork blocks step faster that way.
+bool sweep_pays(int dim, int nwork);
+cudaError_t launch_sweep_update(Launch const &L, double const *U0, double *Uout, double const *F,
+                                long long flux_item_stride, long long dir_stride,
+                                int const *nbr26, CaseState const *cases, int stage);
 
 // One SSP-RK3 stage of every work item by pencil sweeps (engine fast path):
 // the faces of each line of cells along x, then y, then z, with the

@@ -96,14 +96,20 @@ __device__ __forceinline__ void stage_update_cell(double const *Uin, double cons
   interior_coords<DIM>(t, i, j, k);
   int const c = G::cell(i + G::fic(0), j + G::fic(1), k + G::fic(2));
   size_t const base = (size_t)slot * G::BLOCK_DOUBLES + c;
+  // every load before the first store: Uout may alias U0, so the compiler would
+  // keep each field's loads behind the previous field's store
+  double rhs[G::NE], u[G::NE], u0[G::NE];
 #pragma unroll
   for (int f = 0; f < G::NE; ++f) {
     double const *fx = Fb + f * G::FACES;
-    double const rhs = 0.0 + divergence<DIM>(fx, fx + dstride, fx + 2 * dstride, i, j, k,
-                                             one_cell_size);
+    rhs[f] = 0.0 + divergence<DIM>(fx, fx + dstride, fx + 2 * dstride, i, j, k, one_cell_size);
     size_t const x = base + (size_t)f * G::CELLS;
-    Uout[x] = rk_apply(rk, Uin[x], rk.first ? 0.0 : U0[x], rhs);
+    u[f] = Uin[x];
+    u0[f] = rk.first ? 0.0 : U0[x];
   }
+#pragma unroll
+  for (int f = 0; f < G::NE; ++f)
+    Uout[base + (size_t)f * G::CELLS] = rk_apply(rk, u[f], u0[f], rhs[f]);
 }
 
 __device__ __forceinline__ unsigned ld_acquire_u32(unsigned const *p) {
