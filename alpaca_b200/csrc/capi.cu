@@ -156,7 +156,7 @@ int alp_convective_fluxes(int dim, const alp_scheme *scheme, const alp_material 
   L.opt = scheme_options(scheme);
   if (int rc = stateless_glf(L)) return rc;
   long long const stride = (long long)(dim + 2) * faces_of(dim);
-  for (int d = 0; d < dim; ++d) ALP_CUDA(launch_face_flux(L, d, F[d], stride, true));
+  ALP_CUDA(launch_face_flux(L, F, stride, true));
   return ALP_OK;
 }
 
@@ -183,7 +183,8 @@ int alp_space_rhs(int dim, const alp_scheme *scheme, const alp_material *mat,
   if (int rc = stateless_glf(L)) return rc;
   long long const dstride = (long long)(dim + 2) * faces_of(dim);
   long long const stride = dstride * dim;
-  for (int d = 0; d < dim; ++d) ALP_CUDA(launch_face_flux(L, d, F + d * dstride, stride, false));
+  double *const Fd[3] = {F, F + dstride, F + 2 * dstride};
+  ALP_CUDA(launch_face_flux(L, Fd, stride, false));
   ALP_CUDA(launch_divergence(L, F, stride, dstride, d_rhs));
   return ALP_OK;
 }

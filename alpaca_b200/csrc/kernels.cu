@@ -18,6 +18,14 @@ namespace {
 // divergence, stage update
 // ---------------------------------------------------------------------------
 
+// Right-hand side of every cell of the blocks: zero in the halos
+// (space_solver.cpp:58-70), the flux divergence inside. A CTA takes
+// kDivergenceCells consecutive cells of one block and the threads walk its
+// fields, so that the writes are the only pass over the buffer and a call of a
+// few blocks still fills the chip.
+// 125 blocks: 68 us with one CTA per block zeroing, then filling it.
+constexpr int kDivergenceCells = 512;
+
 template <int DIM>
 __global__ void __launch_bounds__(256)
 divergence_kernel(int const *__restrict__ work, BlockMeta const *__restrict__ meta, BlockMeta def,
@@ -27,25 +35,26 @@ divergence_kernel(int const *__restrict__ work, BlockMeta const *__restrict__ me
   int const item = blockIdx.x;
   int const slot = slot_of(work, item);
   double *rb = rhs + (size_t)slot * G::BLOCK_DOUBLES;
-  // zero every cell (space_solver.cpp:58-70), then write the interior
-  for (int x = threadIdx.x; x < G::BLOCK_DOUBLES; x += blockDim.x) rb[x] = 0.0;
-  __syncthreads();
   BlockMeta const bm = meta ? meta[slot] : def;
   double const ocs = inv(bm.cell_size);
   double const *Fb = F + (long long)item * stride;
-  for (int t = threadIdx.x; t < G::INTERIOR; t += blockDim.x) {
-    int i, j, k;
-    interior_coords<DIM>(t, i, j, k);
-    int const c = G::cell(i + G::fic(0), j + G::fic(1), k + G::fic(2));
+  int const end = min(G::CELLS, (int)(blockIdx.y + 1) * kDivergenceCells);
+  for (int x = blockIdx.y * kDivergenceCells + threadIdx.x; x < end; x += blockDim.x) {
+    int const k = x % G::TCZ - G::fic(2), j = (x / G::TCZ) % G::TCY - G::fic(1);
+    int const i = x / (G::TCZ * G::TCY) - G::fic(0);
+    bool const in = (unsigned)i < (unsigned)G::ICX && (unsigned)j < (unsigned)G::ICY &&
+                    (unsigned)k < (unsigned)G::ICZ;
 #pragma unroll
     for (int f = 0; f < G::NE; ++f) {
-      double const *fx = Fb + f * G::FACES;
-      rb[f * G::CELLS + c] =
-          0.0 + divergence<DIM>(fx, fx + dstride, fx + 2 * dstride, i, j, k, ocs);
+      double v = 0.0;
+      if (in) {
+        double const *fx = Fb + f * G::FACES;
+        v = 0.0 + divergence<DIM>(fx, fx + dstride, fx + 2 * dstride, i, j, k, ocs);
+      }
+      rb[f * G::CELLS + x] = v;
     }
   }
 }
-
 
 // Uin: stage input, U0: state at the start of the step, Uout: stage output.
 // Uout may alias U0 (each cell is read and written by the same thread) but
@@ -96,55 +105,73 @@ rk_stage_rhs_kernel(double *__restrict__ U, double *__restrict__ U0,
 
 // Same-level halo regions (communication_types.h:45-132): for direction offset
 // o = +1 the halo [HS+IC, TC) takes the neighbour's [HS, 2HS); o = -1 the halo
-// [0, HS) takes the neighbour's [IC, IC+HS); o = 0 spans the interior.
+// [0, HS) takes the neighbour's [IC, IC+HS); o = 0 spans the interior. A halo
+// cell's offset follows from its coordinates, and its source is the cell 16
+// further inside along the offset. A CTA fills the halo cells of one x plane of
+// one block (3D; the whole block in 1D and 2D), all fields, in storage order,
+// so the stores are whole rows; halos of domain faces are left to
+// zero_gradient_kernel. 125 blocks of 5 fields: 40 us with one CTA per region
+// (26 of them, 4 cells wide along z) and the extents divided at run time.
 template <int DIM>
 __global__ void __launch_bounds__(256)
 halo_region_kernel(double *__restrict__ U, int const *__restrict__ work,
                    int const *__restrict__ nbr26, BlockMeta const *__restrict__ meta,
                    CaseState const *__restrict__ cases, int faces_only, int nfields) {
   using G = Geo<DIM>;
+  constexpr int PLANES = DIM == 3 ? TC : 1;
+  // cells of an interior 3D plane that are halo: 8 whole rows, 8 cells of the others
+  constexpr int ROWS = 2 * HS * TC, RING = ROWS + 2 * HS * IC;
   int const item = blockIdx.x;
   int const slot = slot_of(work, item);
   if (cases && meta && !(cases[meta[slot].case_id].dt > 0.0)) return;
-  // blockIdx.y enumerates the 26 (or 2*DIM) regions
-  int o;
-  if (faces_only) {
-    int const face = blockIdx.y;  // W,E,S,N,B,T
-    int off[3] = {0, 0, 0};
-    off[face / 2] = (face & 1) ? 1 : -1;
-    o = (off[0] + 1) * 9 + (off[1] + 1) * 3 + (off[2] + 1);
-  } else {
-    o = blockIdx.y < 13 ? blockIdx.y : blockIdx.y + 1;
-  }
-  int const off[3] = {o / 9 - 1, (o / 3) % 3 - 1, o % 3 - 1};
-  for (int d = DIM; d < 3; ++d)
-    if (off[d] != 0) return;
-  int const n = nbr26[(size_t)slot * 26 + (o < 13 ? o : o - 1)];
-  if (n < 0) return;  // domain face: zero gradient below
-  int lo[3], ext[3], src[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    if (d >= DIM) {
-      lo[d] = 0; ext[d] = 1; src[d] = 0;
-    } else if (off[d] == 0) {
-      lo[d] = HS; ext[d] = IC; src[d] = HS;
-    } else if (off[d] > 0) {
-      lo[d] = HS + IC; ext[d] = HS; src[d] = HS;
-    } else {
-      lo[d] = 0; ext[d] = HS; src[d] = IC;
-    }
-  }
-  int const cells = ext[0] * ext[1] * ext[2];
+  __shared__ int nb[27];
+  if (threadIdx.x < 27)
+    nb[threadIdx.x] = threadIdx.x == 13 ? -1
+                                        : nbr26[(size_t)slot * 26 + threadIdx.x - (threadIdx.x > 13)];
+  __syncthreads();
+  int const plane = PLANES > 1 ? blockIdx.y : 0;
+  bool const ring = PLANES > 1 && plane >= HS && plane < HS + IC;
+  int const count = ring ? RING : G::CELLS / PLANES;
   double *dst = U + (size_t)slot * nfields * G::CELLS;
-  double const *sb = U + (size_t)n * nfields * G::CELLS;
-  for (int x = threadIdx.x; x < cells * nfields; x += blockDim.x) {
-    int const f = x / cells;
-    int const r = x - f * cells;
-    int const kk = r % ext[2];
-    int const jj = (r / ext[2]) % ext[1];
-    int const ii = r / (ext[2] * ext[1]);
-    dst[f * G::CELLS + G::cell(lo[0] + ii, lo[1] + jj, lo[2] + kk)] =
-        sb[f * G::CELLS + G::cell(src[0] + ii, src[1] + jj, src[2] + kk)];
+  for (int t = threadIdx.x; t < count; t += blockDim.x) {
+    int c[3];
+    if (ring) {
+      c[0] = plane;
+      if (t < ROWS) {
+        int const r = t / TC;
+        c[1] = r < HS ? r : r + IC;
+        c[2] = t - r * TC;
+      } else {
+        int const r = (t - ROWS) / (2 * HS), q = (t - ROWS) % (2 * HS);
+        c[1] = HS + r;
+        c[2] = q < HS ? q : q + IC;
+      }
+    } else {
+      c[2] = t % G::TCZ;
+      c[1] = (t / G::TCZ) % G::TCY;
+      c[0] = PLANES > 1 ? plane : t / (G::TCZ * G::TCY);
+    }
+    int o = 0, nonzero = 0, src[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      int const off = d >= DIM ? 0 : (c[d] < HS ? -1 : (c[d] >= HS + IC ? 1 : 0));
+      o = 3 * o + off + 1;
+      nonzero += off != 0;
+      src[d] = c[d] - IC * off;
+    }
+    int const n = nb[o];
+    if (n < 0 || (faces_only && nonzero != 1)) continue;  // interior, domain face, or not asked for
+    double const *sb = U + (size_t)n * nfields * G::CELLS + G::cell(src[0], src[1], src[2]);
+    double *db = dst + G::cell(c[0], c[1], c[2]);
+    int f = 0;
+    for (; f + 5 <= nfields; f += 5) {  // loads first: the stores may alias them
+      double v[5];
+#pragma unroll
+      for (int q = 0; q < 5; ++q) v[q] = sb[(f + q) * G::CELLS];
+#pragma unroll
+      for (int q = 0; q < 5; ++q) db[(f + q) * G::CELLS] = v[q];
+    }
+    for (; f < nfields; ++f) db[f * G::CELLS] = sb[f * G::CELLS];
   }
 }
 
@@ -231,6 +258,11 @@ prime_states_kernel(double const *__restrict__ U, int const *__restrict__ work,
   }
 }
 
+// CTAs per block of the signal speed: four in 3D, four cells to a thread. 64
+// blocks took 16.6 us with one CTA per block (a chain of 16 loads and square
+// roots per thread).
+__host__ __device__ constexpr int signal_parts(int dim) { return dim == 3 ? 4 : 1; }
+
 // Signal speed of ComputeTimestepSize (modular_algorithm_assembler.cpp:1840-1870):
 // max over interior cells of ConsistencyManagedSum(|u_d| + c).
 template <int DIM>
@@ -246,9 +278,12 @@ signal_speed_kernel(double const *__restrict__ U, int const *__restrict__ work,
   double const *ub = U + (size_t)slot * G::BLOCK_DOUBLES;
   double smax = 0.0;
   int bad = 0;
-  for (int t = threadIdx.x; t < G::INTERIOR; t += blockDim.x) {
+  constexpr int PARTS = signal_parts(DIM);
+  int const first = blockIdx.y * (G::INTERIOR / PARTS);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < G::INTERIOR / PARTS; t += blockDim.x) {
     int i, j, k;
-    interior_coords<DIM>(t, i, j, k);
+    interior_coords<DIM>(first + t, i, j, k);
     int const x = G::cell(i + G::fic(0), j + G::fic(1), k + G::fic(2));
     double c[G::NE];
 #pragma unroll
@@ -358,7 +393,8 @@ int interior_of(int dim) { return dim == 3 ? 4096 : (dim == 2 ? 256 : 16); }
 cudaError_t launch_divergence(Launch const &L, double const *F, long long stride,
                               long long dstride, double *rhs) {
   if (L.nwork <= 0) return cudaSuccess;
-  dim3 grid(L.nwork);
+  int const cells = 24 * (L.dim > 1 ? 24 : 1) * (L.dim > 2 ? 24 : 1);
+  dim3 grid(L.nwork, (cells + kDivergenceCells - 1) / kDivergenceCells);
   switch (L.dim) {
     case 1: divergence_kernel<1><<<grid, 256, 0, L.stream>>>(L.work, L.meta, L.def, F, stride, dstride, rhs); break;
     case 2: divergence_kernel<2><<<grid, 256, 0, L.stream>>>(L.work, L.meta, L.def, F, stride, dstride, rhs); break;
@@ -401,8 +437,7 @@ cudaError_t launch_rk_stage_rhs(int dim, double *U, double *U0, double const *rh
 cudaError_t launch_halo(Launch const &L, int const *nbr26, bool faces_only, int nfields,
                         CaseState const *cases) {
   if (L.nwork <= 0) return cudaSuccess;
-  int const regions = faces_only ? 2 * L.dim : 26;
-  dim3 g1(L.nwork, regions), g2(L.nwork);
+  dim3 g1(L.nwork, L.dim == 3 ? TC : 1), g2(L.nwork);
   int const fo = faces_only ? 1 : 0;
   switch (L.dim) {
     case 1:
@@ -437,7 +472,7 @@ cudaError_t launch_prime_states(Launch const &L, double *P) {
 
 cudaError_t launch_signal_speed(Launch const &L, CaseState *cases, unsigned long long *out) {
   if (L.nwork <= 0) return cudaSuccess;
-  dim3 grid(L.nwork);
+  dim3 grid(L.nwork, signal_parts(L.dim));
   switch (L.dim) {
     case 1: signal_speed_kernel<1><<<grid, 256, 0, L.stream>>>(L.U, L.work, L.meta, L.def, cases, out); break;
     case 2: signal_speed_kernel<2><<<grid, 256, 0, L.stream>>>(L.U, L.work, L.meta, L.def, cases, out); break;

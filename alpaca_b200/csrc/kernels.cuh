@@ -71,15 +71,15 @@ cudaError_t launch_glf_maxima(Launch const &L, unsigned long long *glf, int ncas
 // The library's slot for the stateless calls (one case, id 0).
 unsigned long long *glf_stateless_slot();
 
-// Face fluxes of direction `dir` for every work item into
-// F[item * flux_item_stride + field * FACES + face] (reference flux-array
+// Face fluxes of every direction d of every work item into
+// F[d][item * flux_item_stride + field * FACES + face] (reference flux-array
 // layout). accumulate: += (drop-in contract), else = (zero for skipped faces).
-cudaError_t launch_face_flux(Launch const &L, int dir, double *F, long long flux_item_stride,
-                             bool accumulate, int block_threads = 0);
+cudaError_t launch_face_flux(Launch const &L, double *const F[3], long long flux_item_stride,
+                             bool accumulate);
 
 // SpaceSolver right-hand side: rhs (reference layout, all cells) = 0, interior
 // = consistency-managed flux divergence / cell size. F as written by
-// launch_face_flux for each direction at F + dir * dir_stride.
+// launch_face_flux with direction d at F + d * dir_stride.
 cudaError_t launch_divergence(Launch const &L, double const *F, long long flux_item_stride,
                               long long dir_stride, double *rhs);
 
