@@ -584,7 +584,11 @@ jump_average_kernel(int const *__restrict__ fine, JumpRec const *__restrict__ re
 // JumpFluxAdjustment of the coarse leaves that finished a step: cells next to
 // a refined neighbour get - CMS(coarse) + CMS(fine) of their face sums divided
 // by the cell size (signs: +1 on West / South / Bottom faces, -1 on East /
-// North / Top), then the sums are reset.
+// North / Top), then the sums are reset. One CTA per (leaf, field); its threads
+// take the cells of one jump face after the other, and a cell on several of
+// them is taken with the first. Few leaves are corrected at once, so the kernel
+// is a chain of latencies: 24 leaves of the three-level step took 130 us with
+// one CTA per leaf scanning all its cells.
 template <int DIM>
 __global__ void __launch_bounds__(256)
 jump_correct_kernel(CorrectRec const *__restrict__ corr, JumpRec const *__restrict__ recs,
@@ -592,49 +596,52 @@ jump_correct_kernel(CorrectRec const *__restrict__ corr, JumpRec const *__restri
                     BlockMeta const *__restrict__ meta, CaseState const *__restrict__ cu) {
   using G = Geo<DIM>;
   using FC = FaceCells<DIM>;
-  CorrectRec const cr = corr[blockIdx.x];
+  CorrectRec const &cr = corr[blockIdx.x];
   if (!(cu[cr.level].dt > 0.0)) return;
+  int const e = blockIdx.y;
   double const ocs = 1.0 / meta[cr.slot].cell_size;
-  double *ub = U + (size_t)cr.slot * G::BLOCK_DOUBLES;
-  for (int t = threadIdx.x; t < G::INTERIOR; t += blockDim.x) {
-    int a[3];
-    interior_coords<DIM>(t, a[0], a[1], a[2]);
-    bool touched = false;
+  double *ub = U + (size_t)cr.slot * G::BLOCK_DOUBLES + e * G::CELLS;
+  double *J[2 * DIM], *A[2 * DIM];
 #pragma unroll
-    for (int loc = 0; loc < 2 * DIM; ++loc) {
-      int const d = loc / 2;
-      touched |= cr.rec[loc] >= 0 && a[d] == ((loc % 2) ? 0 : IC - 1);
-    }
-    if (!touched) continue;
-    int const cell = G::cell(a[0] + G::fic(0), a[1] + G::fic(1), a[2] + G::fic(2));
-    for (int e = 0; e < G::NE; ++e) {
-      double cf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ff[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int loc = 0; loc < 2 * DIM; ++loc) {
-        int const d = loc / 2, high = (loc % 2) == 0;
-        int const ri = cr.rec[loc];
-        if (ri < 0 || a[d] != (high ? IC - 1 : 0)) continue;
-        int const t1 = FC::t1(d), t2 = FC::t2(d);
-        int const x = e * IC * IC + a[t1] * IC + a[t2];
-        double const dir = high ? -1.0 : 1.0;
-        cf[loc] = jbuf[(size_t)ri * G::NE * IC * IC + x] * ocs * dir;
-        ff[loc] = acc[(size_t)recs[ri].acc * G::NE * IC * IC + x] * ocs * dir;
-      }
-      double &u = ub[e * G::CELLS + cell];
-      u -= cms3(cf[0] + cf[1], cf[2] + cf[3], cf[4] + cf[5]);
-      u += cms3(ff[0] + ff[1], ff[2] + ff[3], ff[4] + ff[5]);
-    }
-  }
-  __syncthreads();
   for (int loc = 0; loc < 2 * DIM; ++loc) {
     int const ri = cr.rec[loc];
-    if (ri < 0) continue;
-    double *J = jbuf + (size_t)ri * G::NE * IC * IC;
-    double *A = acc + (size_t)recs[ri].acc * G::NE * IC * IC;
-    for (int x = threadIdx.x; x < G::NE * IC * IC; x += blockDim.x) {
-      J[x] = 0.0;
-      A[x] = 0.0;
+    size_t const row = ((size_t)G::NE * (ri < 0 ? 0 : ri) + e) * IC * IC;
+    J[loc] = ri < 0 ? nullptr : jbuf + row;
+    A[loc] = ri < 0 ? nullptr : acc + ((size_t)G::NE * recs[ri].acc + e) * IC * IC;
+  }
+#pragma unroll
+  for (int first = 0; first < 2 * DIM; ++first) {
+    if (!J[first]) continue;
+    int const df = first / 2, n2f = FC::n(FC::t2(df));
+    int const t = threadIdx.x;
+    if (t >= FC::n(FC::t1(df)) * n2f) continue;
+    int a[3] = {0, 0, 0};
+    a[df] = (first % 2) ? 0 : IC - 1;
+    a[FC::t1(df)] = t / n2f;
+    a[FC::t2(df)] = t % n2f;
+    bool done = false;
+    double cf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ff[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int loc = 0; loc < 2 * DIM; ++loc) {
+      int const d = loc / 2, high = (loc % 2) == 0;
+      if (!J[loc] || a[d] != (high ? IC - 1 : 0)) continue;
+      if (loc < first) done = true;
+      int const x = a[FC::t1(d)] * IC + a[FC::t2(d)];
+      double const dir = high ? -1.0 : 1.0;
+      cf[loc] = J[loc][x] * ocs * dir;
+      ff[loc] = A[loc][x] * ocs * dir;
     }
+    if (done) continue;
+    double &u = ub[G::cell(a[0] + G::fic(0), a[1] + G::fic(1), a[2] + G::fic(2))];
+    u -= cms3(cf[0] + cf[1], cf[2] + cf[3], cf[4] + cf[5]);
+    u += cms3(ff[0] + ff[1], ff[2] + ff[3], ff[4] + ff[5]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int loc = 0; loc < 2 * DIM; ++loc) {
+    if (!J[loc]) continue;
+    J[loc][threadIdx.x] = 0.0;  // IC * IC threads
+    A[loc][threadIdx.x] = 0.0;
   }
 }
 
@@ -902,9 +909,9 @@ struct alp_levels {
       }
       if (ncorr > 0) {
         switch (dim) {
-          case 1: jump_correct_kernel<1><<<ncorr, 256, 0, stream>>>(jcorr, jrecs, jbuf, jacc, U, meta, cu); break;
-          case 2: jump_correct_kernel<2><<<ncorr, 256, 0, stream>>>(jcorr, jrecs, jbuf, jacc, U, meta, cu); break;
-          default: jump_correct_kernel<3><<<ncorr, 256, 0, stream>>>(jcorr, jrecs, jbuf, jacc, U, meta, cu); break;
+          case 1: jump_correct_kernel<1><<<dim3(ncorr, ne), 256, 0, stream>>>(jcorr, jrecs, jbuf, jacc, U, meta, cu); break;
+          case 2: jump_correct_kernel<2><<<dim3(ncorr, ne), 256, 0, stream>>>(jcorr, jrecs, jbuf, jacc, U, meta, cu); break;
+          default: jump_correct_kernel<3><<<dim3(ncorr, ne), 256, 0, stream>>>(jcorr, jrecs, jbuf, jacc, U, meta, cu); break;
         }
         ALP_CUDA(cudaGetLastError());
       }
