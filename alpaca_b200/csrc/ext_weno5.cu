@@ -1,0 +1,4 @@
+// Kernels of the run-time selected schemes with the WENO5 stencil.
+#include "ext_kernels.cuh"
+
+template struct alp::ExtKernels<alp::ST_WENO5>;

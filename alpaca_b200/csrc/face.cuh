@@ -78,7 +78,7 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
   constexpr int C = W / 2 - 1;  // the face's left cell i in the stencil
 
   if constexpr (SCHEME == FV_CHAR || SCHEME == FS_ROE) {
-    if constexpr (ALP_FAST && sizeof(T) == 8 && P::is_default) {
+    if constexpr (ALP_FAST && sizeof(T) == 8 && P::FAST_FRAME) {
       // the factored characteristic frame on the five differences of the six
       // cells (each side's reconstruction is its own cell plus an increment)
       auto const ct = char_cell<DIM, DIR>(eos, cons[C]);
@@ -98,7 +98,7 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
         }
         double il[NE], ir[NE];
 #pragma unroll
-        for (int n = 0; n < NE; ++n) weno5_increments(G[n], char_eps<DIM>(r, n), il[n], ir[n]);
+        for (int n = 0; n < NE; ++n) pol.increments(G[n], char_scale<DIM>(r, n), il[n], ir[n]);
         double cm[NE], cp[NE];
         char_restore<DIM, DIR>(r, cons[C], il, 1.0, cm);
         char_restore<DIM, DIR>(r, cons[C + 1], ir, -1.0, cp);
@@ -106,13 +106,15 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
         auto const sm = recon_state<DIM, DIR>(eos, cm);
         auto const sp = recon_state<DIM, DIR>(eos, cp);
         if (!(sm.p > -B) || !(sp.p > -B)) valid = false;
-        hllc<DIM, DIR, double>(eos, cm, cp, sm.p, sp.p, sm.v, sp.v, sm.one, sp.one, fd);
+        pol.template riemann<DIM, DIR, double>(eos, cm, cp, sm.p, sp.p, sm.v, sp.v, sm.one, sp.one,
+                                               fd);
       } else {
         // Roe flux-vector splitting: the split fluxes f +/- alpha u of each
         // wave from the projected differences of f and u. The mean of the two
         // reconstructions is (f_i + f_i+1) / 2 plus R times half of
         // (left increment - right increment - alpha L (u_i+1 - u_i)).
-        double const al[3] = {fabs(r.up - r.c), fabs(r.up), fabs(r.up + r.c)};
+        double al[3];
+        pol.frame_eigenvalues(eos, r, ct, cn, cons[C][MASS], cons[C + 1][MASS], al);
         double A[NE][5], N[NE][5], w[NE];
         double fa[NE], fb[NE], fi[NE];
         phys_flux<DIM, DIR>(eos, cons[0], fa);
@@ -150,7 +152,7 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
           double l, q;
           A[n][4] = 0.0;
           N[n][0] = 0.0;
-          weno5_increments_two(A[n], N[n], char_eps<DIM>(r, n), l, q);
+          pol.increments_two(A[n], N[n], char_scale<DIM>(r, n), l, q);
           w[n] = 0.5 * ((l - q) - w[n]);
         }
         char_restore<DIM, DIR>(r, fi, w, 1.0, fd);
@@ -382,7 +384,7 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
     double prim[W][NE];
 #pragma unroll
     for (int m = 0; m < W; ++m) {
-      if constexpr (ALP_FAST && P::is_default) {
+      if constexpr (ALP_FAST) {
         // velocities, then the pressure with the kinetic energy u . m / 2
         prim[m][RHO] = cons[m][MASS];
         double const one = inv(cons[m][MASS]);
@@ -441,12 +443,21 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
       T pm[NE], pp[NE];
 #pragma unroll
       for (int n = 0; n < NE; ++n) {
-        T arr[W];
+        if constexpr (ALP_FAST && P::FAST_FRAME) {
+          double G[5], l, r;
 #pragma unroll
-        for (int m = 0; m < W; ++m) arr[m] = T(prim[m][n]);
-        pol.pair(arr, pm[n], pp[n]);
+          for (int m = 0; m < 5; ++m) G[m] = prim[m + 1][n] - prim[m][n];
+          pol.increments(G, 1.0, l, r);
+          pm[n] = prim[C][n] + l;
+          pp[n] = prim[C + 1][n] - r;
+        } else {
+          T arr[W];
+#pragma unroll
+          for (int m = 0; m < W; ++m) arr[m] = T(prim[m][n]);
+          pol.pair(arr, pm[n], pp[n]);
+        }
       }
-      if constexpr (ALP_FAST && sizeof(T) == 8 && P::is_default) {
+      if (ALP_FAST && pol.default_riemann()) {
         // the upwind side's conservatives alone (hllc_upwind)
         if (!(pm[RHO] > DBL_EPSILON) || !(pp[RHO] > DBL_EPSILON)) valid = false;
         if (!(pm[PRES] > -B) || !(pp[PRES] > -B)) valid = false;

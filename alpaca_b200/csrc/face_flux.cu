@@ -10,9 +10,6 @@ namespace {
 // the buffer); direction blockIdx.z goes to F.d[blockIdx.z]. A call with one
 // block has 34 CTAs per direction: side by side they take 6 us, one launch
 // after the other 17 us.
-struct FluxPtrs {
-  double *d[3];
-};
 template <int DIM, int SCHEME, typename T, bool ACCUM>
 __global__ void __launch_bounds__(128, FaceOccupancy<DIM, SCHEME, T>::min_ctas)
 face_flux_kernel(double const *__restrict__ U, int const *__restrict__ work,
@@ -75,13 +72,11 @@ cudaError_t face_flux_dim(Launch const &L, FluxPtrs const &F, long long stride) 
   constexpr int threads = 128;
   int const chunks = (FaceMap<DIM, 0>::COUNT + threads - 1) / threads;
   if ((long long)L.nwork * chunks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  if (!L.opt.is_default()) {
-    for (int d = 0; d < DIM; ++d)
-      if (cudaError_t e = face_flux_ext(L, d, ACC, dim3(L.nwork, chunks), F.d[d], stride, threads))
-        return e;
-    return cudaSuccess;
-  }
   dim3 const grid((unsigned)(L.nwork * chunks), 1, DIM);
+  if (!L.opt.is_default())
+    return with_stencil(L, [&](auto k) {
+      return decltype(k)::face(L, ACC, grid, chunks, F, stride, threads);
+    });
   switch (L.scheme) {
     case FV_CHAR:
       face_flux_kernel<DIM, FV_CHAR, T, ACC>
@@ -128,13 +123,14 @@ template <int DIM, typename T>
 cudaError_t face_flux_all_t(Launch const &L, int const *nbr26, CaseState const *cases, double *F,
                             long long stride, long long dstride, int threads, int dirs) {
   int const count = (IC + 1) * (DIM > 1 ? IC : 1) * (DIM > 2 ? IC : 1);
-  dim3 grid(L.nwork, (count + threads - 1) / threads, dirs);
-  if (!L.opt.is_default())
-    return face_flux_all_ext(L, grid, nbr26, cases, F, stride, dstride, threads);
   // items x chunks < 2^31 for up to 2^31 / 68 items (64-thread chunks)
   int const chunks = (count + threads - 1) / threads;
   if ((long long)L.nwork * chunks > 0x7fffffffLL) return cudaErrorInvalidValue;
   dim3 const g2((unsigned)(L.nwork * chunks), 1, dirs);
+  if (!L.opt.is_default())
+    return with_stencil(L, [&](auto k) {
+      return decltype(k)::face_all(L, g2, chunks, nbr26, cases, F, stride, dstride, threads);
+    });
   switch (L.scheme) {
     case FV_CHAR:
       face_flux_all_kernel<DIM, FV_CHAR, T><<<g2, threads, 0, L.stream>>>(L.U, L.work, L.meta, nbr26, cases, F, stride, dstride, chunks, L.items);

@@ -189,19 +189,5 @@ __device__ __forceinline__ void face_flux(double const *__restrict__ U,
   write_flux<DIM, DIR, ACCUM>(F, item, stride, a, p1, p2, valid, fd);
 }
 
-// The run-time selected schemes read 6-cell stencils (i-2 .. i+3), or 8-cell
-// stencils (i-3 .. i+4) when the stencil is WENO7; the narrower stencils use
-// the middle cells. The 8-wide instantiation holds 33 % more stencil state, so
-// the launchers pick it only for WENO7.
-inline bool ext_wide(SchemeOptions const &o) { return o.stencil == ST_WENO7; }
-
-// The policy of one block: the GlobalLaxFriedrichs wave speeds of its case.
-__device__ __forceinline__ ExtPolicy block_policy(ExtPolicy pol, BlockMeta const &bm,
-                                                  unsigned long long const *glf) {
-  if (glf && pol.o.splitting == FSP_GLF)
-    for (int k = 0; k < 3; ++k) pol.glf[k] = __longlong_as_double(glf[4 * bm.case_id + k]);
-  return pol;
-}
-
 }  // namespace
 }  // namespace alp

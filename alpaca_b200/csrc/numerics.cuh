@@ -745,10 +745,10 @@ __device__ __forceinline__ void char_project(CharFrame<DIM> const &r, double con
   ch[DIM + 1] = fma(r.one_c, Dp, s);
 }
 
-// eps of the reconstruction of wave n in these scales.
+// Square of the factor on the characteristic values of wave n in these scales.
 template <int DIM>
-__device__ __forceinline__ double char_eps(CharFrame<DIM> const &r, int n) {
-  return n == 0 || n == DIM + 1 ? 4.0e-6 : (n == DIM ? 1.0e-6 : 1.0e-6 * r.rho2);
+__device__ __forceinline__ double char_scale(CharFrame<DIM> const &r, int n) {
+  return n == 0 || n == DIM + 1 ? 4.0 : (n == DIM ? 1.0 : r.rho2);
 }
 
 // base + sgn (the conserved difference whose scaled characteristic values are ch).

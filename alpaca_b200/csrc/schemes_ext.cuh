@@ -96,6 +96,92 @@ __device__ __forceinline__ double weno3_core(double v1, double v2, double v3) {
   return w1 * (-1.0 / 2.0 * v1 + 3.0 / 2.0 * v2) + w2 * (1.0 / 2.0 * v2 + 1.0 / 2.0 * v3);
 }
 
+// Fast-build forms of the six-cell stencils: num / (FACTOR den) is the increment
+// from the centre cell v3 to the reconstructed value, from the first differences
+// g1..g4 of v1..v5 (weno5_frac's candidates and indicators; eps scaled by the
+// square of the caller's factor on the differences).
+template <int ST> struct StencilFrac;
+template <> struct StencilFrac<ST_WENO5> {
+  static constexpr double FACTOR = 6.0, EPS = 1.0e-6;
+  __device__ __forceinline__ static Weno5Frac make(double g1, double g2, double g3, double g4,
+                                                   double eps) {
+    double const d1 = g2 - g1, d2 = g3 - g2, d3 = g4 - g3;
+    return weno5_frac(g2, g3, d1, d3, weno5_q(d1, eps), weno5_q(d2, eps), weno5_q(d3, eps));
+  }
+};
+// alpha_k = d_k (1 + tau / s_k), s_k = beta_k + eps, times s1 s2 s3
+template <> struct StencilFrac<ST_WENO5Z> {
+  static constexpr double FACTOR = 6.0, EPS = DBL_EPSILON;
+  __device__ __forceinline__ static Weno5Frac make(double g1, double g2, double g3, double g4,
+                                                   double eps) {
+    double const d1 = g2 - g1, d2 = g3 - g2, d3 = g4 - g3;
+    double const a = g2 + d1, b = g3 - d3;
+    double const s1 = fma(g2, a, weno5_q(d1, eps)), s2 = fma(g2, g3, weno5_q(d2, eps));
+    double const s3 = fma(g3, b, weno5_q(d3, eps));
+    double const tau = fabs(s1 - s3);
+    double const a1 = (s1 + tau) * (s2 * s3);
+    double const a2 = 6.0 * ((s2 + tau) * (s1 * s3));
+    double const a3 = 3.0 * ((s3 + tau) * (s1 * s2));
+    return {fma(a3, fma(2.0, g3, b), fma(a2, fma(2.0, g3, g2), a1 * fma(2.0, a, g2))),
+            a1 + a2 + a3};
+  }
+};
+// x_k = 1 + tau / s_k, alpha_k = x_k^6, cut off below 1e-5 of their sum
+template <> struct StencilFrac<ST_TENO5> {
+  static constexpr double FACTOR = 6.0, EPS = DBL_EPSILON;
+  __device__ __forceinline__ static Weno5Frac make(double g1, double g2, double g3, double g4,
+                                                   double eps) {
+    double const d1 = g2 - g1, d2 = g3 - g2, d3 = g4 - g3;
+    double const a = g2 + d1, b = g3 - d3;
+    double const s1 = fma(g2, a, weno5_q(d1, eps)), s2 = fma(g2, g3, weno5_q(d2, eps));
+    double const s3 = fma(g3, b, weno5_q(d3, eps));
+    double const tau = fabs(s1 - s3);
+    double const r = inv(s1 * s2 * s3);
+    double x1 = (s1 + tau) * ((s2 * s3) * r), x2 = (s2 + tau) * ((s1 * s3) * r);
+    double x3 = (s3 + tau) * ((s1 * s2) * r);
+    x1 *= x1 * x1;
+    x2 *= x2 * x2;
+    x3 *= x3 * x3;
+    x1 *= x1;
+    x2 *= x2;
+    x3 *= x3;
+    double const cut = 1.0e-5 * (x1 + x2 + x3);
+    double const w1 = x1 < cut ? 0.0 : 1.0, w2 = x2 < cut ? 0.0 : 6.0, w3 = x3 < cut ? 0.0 : 3.0;
+    return {fma(w3, fma(2.0, g3, b), fma(w2, fma(2.0, g3, g2), w1 * fma(2.0, a, g2))),
+            w1 + w2 + w3};
+  }
+};
+// v2 + (t2 g1 + 2 t1 g2) / (2 (t2 + 2 t1)) on the middle three cells, t_k = (g_k^2 + eps)^2
+template <> struct StencilFrac<ST_WENO3> {
+  static constexpr double FACTOR = 2.0, EPS = DBL_EPSILON;
+  __device__ __forceinline__ static Weno5Frac make(double, double g2, double g3, double,
+                                                   double eps) {
+    double const s1 = fma(g2, g2, eps), s2 = fma(g3, g3, eps);
+    double const t1 = 2.0 * (s1 * s1), t2 = s2 * s2;
+    return {fma(t1, g3, t2 * g2), t1 + t2};
+  }
+};
+
+// Increments of both sides of a face (weno5_increments of another stencil):
+// left from the differences A[0..3], right from B[1..4] (one array for both in
+// the finite-volume schemes).
+template <int ST>
+__device__ __forceinline__ void stencil_increments(double const (&A)[5], double const (&B)[5],
+                                                   double scale, double &left, double &right) {
+  if constexpr (ST == ST_FIRST_ORDER) {
+    left = 0.0;
+    right = 0.0;
+  } else {
+    using S = StencilFrac<ST>;
+    double const eps = S::EPS * scale;
+    Weno5Frac const l = S::make(A[0], A[1], A[2], A[3], eps);
+    Weno5Frac const r = S::make(B[4], B[3], B[2], B[1], eps);
+    double const rr = inv((S::FACTOR * l.den) * r.den);
+    left = l.num * (r.den * rr);
+    right = r.num * (l.den * rr);
+  }
+}
+
 // Reconstruction of the 6-cell array a (cells i-2..i+3 around face i+1/2) with
 // UpwindLeft (right = false) or UpwindRight evaluation properties
 // (stencils/apply_wrapper.h:47-57); narrower stencils use the middle cells.
@@ -292,9 +378,30 @@ __device__ __forceinline__ void riemann_ext(int solver, int speeds, Eos const &e
 }
 
 // Scheme policies of face_compute. The default one is the compiled hot path;
-// ExtPolicy dispatches on SchemeOptions at run time (FP64 only).
+// ExtPolicy (FP64 only) has its stencil compiled in and dispatches on the Riemann
+// solver, signal speed and splitting of SchemeOptions at run time: 64 blocks of
+// WENO5-Z took 119 us a launch with the stencil chosen at run time too.
+// FAST_FRAME: the fast build's FP64 face_compute runs on the differences of the
+// stencil (CharFrame), reconstructed by increments / increments_two.
 struct DefaultPolicy {
-  static constexpr bool is_default = true;
+  static constexpr bool FAST_FRAME = true;
+  __device__ __forceinline__ void increments(double const (&G)[5], double scale, double &l,
+                                             double &r) const {
+    weno5_increments(G, 1.0e-6 * scale, l, r);
+  }
+  __device__ __forceinline__ void increments_two(double const (&A)[5], double const (&B)[5],
+                                                 double scale, double &l, double &r) const {
+    weno5_increments_two(A, B, 1.0e-6 * scale, l, r);
+  }
+  __host__ __device__ static constexpr bool default_riemann() { return true; }
+  template <int DIM>
+  __device__ __forceinline__ void frame_eigenvalues(Eos const &, CharFrame<DIM> const &r,
+                                                    CharCell<DIM> const &, CharCell<DIM> const &,
+                                                    double, double, double (&al)[3]) const {
+    al[0] = fabs(r.up - r.c);
+    al[1] = fabs(r.up);
+    al[2] = fabs(r.up + r.c);
+  }
   template <typename T> __device__ __forceinline__ T left(T const (&a)[6]) const {
     return weno5_left(a);
   }
@@ -327,15 +434,52 @@ struct DefaultPolicy {
   }
 };
 
-struct ExtPolicy {
-  static constexpr bool is_default = false;
+template <int ST> struct ExtPolicy {
+  // WENO7 reads eight cells and its indicators are forms in the values themselves
+  static constexpr bool FAST_FRAME = ST != ST_WENO7;
   SchemeOptions o;
   double glf[3] = {0.0, 0.0, 0.0};  // GlobalLaxFriedrichs wave speeds of the block's case
+  __device__ __forceinline__ void increments(double const (&G)[5], double scale, double &l,
+                                             double &r) const {
+    stencil_increments<ST>(G, G, scale, l, r);
+  }
+  __device__ __forceinline__ void increments_two(double const (&A)[5], double const (&B)[5],
+                                                 double scale, double &l, double &r) const {
+    stencil_increments<ST>(A, B, scale, l, r);
+  }
+  __device__ __forceinline__ bool default_riemann() const {
+    return o.riemann == RS_HLLC && o.signal == SS_EINFELDT;
+  }
+  template <int DIM>
+  __device__ __forceinline__ void frame_eigenvalues(Eos const &e, CharFrame<DIM> const &r,
+                                                    CharCell<DIM> const &t, CharCell<DIM> const &n,
+                                                    double rho_t, double rho_n,
+                                                    double (&al)[3]) const {
+    double const phi = 5.0;  // FluxSplittingSettings::low_mach_number_limit_factor
+    if (o.splitting == FSP_GLF) {
+      // the x maxima in every direction (eigendecomposition.h:457-460)
+      for (int k = 0; k < 3; ++k) al[k] = glf[k];
+    } else if (o.splitting == FSP_LLF || o.splitting == FSP_LLF_M) {
+      double ct = tsqrt(eos_cc(e, rho_t, t.p, t.one)), cn = tsqrt(eos_cc(e, rho_n, n.p, n.one));
+      if (o.splitting == FSP_LLF_M) {
+        ct = dmin(phi * fabs(t.up), ct);
+        cn = dmin(phi * fabs(n.up), cn);
+      }
+      al[0] = dmax(fabs(t.up - ct), fabs(n.up - cn));
+      al[1] = dmax(fabs(t.up), fabs(n.up));
+      al[2] = dmax(fabs(t.up + ct), fabs(n.up + cn));
+    } else {
+      double const c = o.splitting == FSP_ROE_M ? dmin(r.c, phi * fabs(r.up)) : r.c;
+      al[0] = fabs(r.up - c);
+      al[1] = fabs(r.up);
+      al[2] = fabs(r.up + c);
+    }
+  }
   template <int N> __device__ __forceinline__ double left(double const (&a)[N]) const {
-    return reconstruct(o.stencil, a, false);
+    return reconstruct(ST, a, false);
   }
   template <int N> __device__ __forceinline__ double right(double const (&a)[N]) const {
-    return reconstruct(o.stencil, a, true);
+    return reconstruct(ST, a, true);
   }
   template <int N>
   __device__ __forceinline__ void pair(double const (&a)[N], double &l, double &r) const {
@@ -353,7 +497,10 @@ struct ExtPolicy {
                                           double const (&cr)[DIM + 2], double pl, double pr,
                                           double vl, double vr, double one_l, double one_r,
                                           double (&flux)[DIM + 2]) const {
-    riemann_ext<DIM, DIR>(o.riemann, o.signal, e, cl, cr, pl, pr, vl, vr, one_l, one_r, flux);
+    if (ALP_FAST && default_riemann())
+      hllc<DIM, DIR, double>(e, cl, cr, pl, pr, vl, vr, one_l, one_r, flux);
+    else
+      riemann_ext<DIM, DIR>(o.riemann, o.signal, e, cl, cr, pl, pr, vl, vr, one_l, one_r, flux);
   }
   // eigendecomposition.h:416-454
   template <int DIM, int DIR, typename T>

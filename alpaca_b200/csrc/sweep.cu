@@ -28,7 +28,10 @@ cudaError_t sweep_t(Launch const &L, double const *U0, double *Uout, double cons
   if (units > 0x7fffffffLL) return cudaErrorInvalidValue;
   int const n = (int)units, grid = (n + kSweepWarps - 1) / kSweepWarps, th = 32 * kSweepWarps;
   if (!L.opt.is_default())
-    return sweep_ext(L, grid, th, U0, Uout, F, stride, dstride, nbr26, cases, stage, rows, n);
+    return with_stencil(L, [&](auto k) {
+      return decltype(k)::sweep(L, grid, th, U0, Uout, F, stride, dstride, nbr26, cases, stage, rows,
+                                n);
+    });
   switch (L.scheme) {
     case FV_CHAR:
       sweep_update_kernel<DIM, FV_CHAR, T><<<grid, th, 0, L.stream>>>(L.U, U0, Uout, L.work, L.meta, nbr26, cases, F, stride, dstride, stage, rows, n);

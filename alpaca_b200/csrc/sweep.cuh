@@ -1,6 +1,6 @@
 // The last direction's faces fused with the stage update, shared by the kernels
 // of the compiled default (sweep.cu) and of the run-time selected schemes
-// (sweep_ext.cu).
+// (ext_kernels.cuh).
 #pragma once
 
 #include "face_kernels.cuh"
@@ -8,14 +8,18 @@
 namespace alp {
 namespace {
 
-// The policy of a sweep's block (block_policy for the run-time selected schemes).
-__device__ __forceinline__ DefaultPolicy sweep_policy(DefaultPolicy const &pol, BlockMeta const &,
+// The policy of one block: for the run-time selected schemes with the
+// GlobalLaxFriedrichs wave speeds of its case.
+__device__ __forceinline__ DefaultPolicy block_policy(DefaultPolicy const &pol, BlockMeta const &,
                                                       unsigned long long const *) {
   return pol;
 }
-__device__ __forceinline__ ExtPolicy sweep_policy(ExtPolicy const &pol, BlockMeta const &bm,
-                                                  unsigned long long const *glf) {
-  return block_policy(pol, bm, glf);
+template <int ST>
+__device__ __forceinline__ ExtPolicy<ST> block_policy(ExtPolicy<ST> pol, BlockMeta const &bm,
+                                                      unsigned long long const *glf) {
+  if (glf && pol.o.splitting == FSP_GLF)
+    for (int k = 0; k < 3; ++k) pol.glf[k] = __longlong_as_double(glf[4 * bm.case_id + k]);
+  return pol;
 }
 
 // The faces of the last direction (z in 3D, y in 2D) and the stage update in one
@@ -50,7 +54,7 @@ __device__ __forceinline__ void sweep_update(double const *Uin, double const *U0
   BlockMeta const bm = meta[slot];
   double const dt = cases[bm.case_id].dt;
   if (!(dt > 0.0)) return;
-  P const pol = sweep_policy(pol0, bm, glf);
+  P const pol = block_policy(pol0, bm, glf);
   double const *Fb = F + (long long)item * stride;
   double const ocs = inv(bm.cell_size);
   RkStage const rk = rk_stage(stage, dt);
