@@ -165,43 +165,41 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
     Roe<T> const r = roe_average<DIM, DIR, T>(eos, pt, pn);
     T ch[2][NE];
     if constexpr (SCHEME == FV_CHAR && sizeof(T) == 4) {
-      // FP32 form: characteristic projection and WENO5 of the increments
-      // U_m - U_i against the face's left cell i (WENO5 is translation
-      // invariant and R L = I), the left cell's state added back in double.
-      // The increments are formed in double and converted once each, for all
-      // five characteristic fields.
-      float du[W][NE];
-#pragma unroll
-      for (int m = 0; m < W; ++m)
-#pragma unroll
-        for (int l = 0; l < NE; ++l) du[m][l] = m == C ? 0.0f : float(cons[m][l] - cons[C][l]);
+      // FP32 form: characteristic projection and WENO5 of the state's variation
+      // (WENO5 is translation invariant and R L = I), the face's left cell added
+      // back in double. The variation is formed in double and converted once.
       T dm[NE], dp[NE];
-      if constexpr (ALP_FAST && W == 6 && C == 2) {
-        // both sides of every characteristic field in packed f32x2 arithmetic
-        // the projection of cells (0, 5) and (1, 4) packed as well; cell 2 is
-        // the face's left cell, whose increment is zero
-        float2 chp[NE], out[NE];
+      if constexpr (ALP_FAST && W == 6) {
+        // the first differences of the six cells, projected and reconstructed
+        // with both sides of the face as the lanes of packed f32x2 arithmetic:
+        // differences 0 and 4, 1 and 3 as pairs, 2 alone
+        float2 x0[NE], x1[NE], chp[NE], out[NE];
+        float x2[NE];
+#pragma unroll
+        for (int l = 0; l < NE; ++l) {
+          x0[l] = make_float2(float(cons[1][l] - cons[0][l]), float(cons[5][l] - cons[4][l]));
+          x1[l] = make_float2(float(cons[2][l] - cons[1][l]), float(cons[4][l] - cons[3][l]));
+          x2[l] = float(cons[3][l] - cons[2][l]);
+        }
 #pragma unroll
         for (int n = 0; n < NE; ++n) {
           T L[NE];
           left_row<DIM, DIR, T>(n, r, L);
-          float2 P0 = make_float2(0.0f, 0.0f), P1 = P0;
-          float u3 = 0.0f;
+          float2 g0 = make_float2(0.0f, 0.0f), g1 = g0;
+          float g2 = 0.0f;
           bool first = true;
 #pragma unroll
           for (int q = 0; q < NE; ++q) {
             int const l = sum_seq<DIM, DIR>(q);
             if (!left_nonzero<DIM, DIR>(n, l)) continue;
             float2 const Ld = dup2(L[l]);
-            float2 const a0 = make_float2(du[0][l], du[5][l]);
-            float2 const a1 = make_float2(du[1][l], du[4][l]);
-            P0 = first ? mul2(Ld, a0) : fma2(Ld, a0, P0);
-            P1 = first ? mul2(Ld, a1) : fma2(Ld, a1, P1);
-            u3 = fmaf(L[l], du[3][l], u3);
+            g0 = first ? mul2(Ld, x0[l]) : fma2(Ld, x0[l], g0);
+            g1 = first ? mul2(Ld, x1[l]) : fma2(Ld, x1[l], g1);
+            g2 = first ? L[l] * x2[l] : fmaf(L[l], x2[l], g2);
             first = false;
           }
-          chp[n] = weno5_packed(P0, P1, make_float2(0.0f, u3), make_float2(u3, 0.0f),
-                                make_float2(P1.y, P1.x));
+          float2 const i = weno5_packed(g0, g1, dup2(g2), make_float2(g1.y, g1.x), 1.0e-6f);
+          chp[n] = make_float2(i.x, g2 - i.y);  // the right cell is g2 beyond the left one
         }
         to_physical_packed<DIM, DIR>(r, chp, out);
 #pragma unroll
@@ -210,6 +208,11 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
           dp[f] = out[f].y;
         }
       } else {
+        float du[W][NE];
+#pragma unroll
+        for (int m = 0; m < W; ++m)
+#pragma unroll
+          for (int l = 0; l < NE; ++l) du[m][l] = m == C ? 0.0f : float(cons[m][l] - cons[C][l]);
 #pragma unroll
         for (int n = 0; n < NE; ++n) {
           T L[NE];
@@ -238,6 +241,15 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
         cp[f] = cons[C][f] + double(dp[f]);
       }
       if (!(cm[MASS] > DBL_EPSILON) || !(cp[MASS] > DBL_EPSILON)) valid = false;
+      if constexpr (ALP_FAST) {
+        auto const sm = recon_state<DIM, DIR>(eos, cm);
+        auto const sp = recon_state<DIM, DIR>(eos, cp);
+        if (!(sm.p > -B) || !(sp.p > -B)) valid = false;
+        hllc_flux<DIM, DIR>(hllc_upwind_mixed(eos, cm[MASS], cp[MASS], sm.p, sp.p, sm.v, sp.v,
+                                              sm.one, sp.one),
+                            cm, cp, fd);
+        return valid;
+      }
       double const one_l = inv(cm[MASS]), one_r = inv(cp[MASS]);
       double const pm = eos_pressure<DIM>(eos, cm[MASS], cm[MOMX], DIM > 1 ? cm[MOMX + (DIM > 1)] : 0.0,
                                           DIM > 2 ? cm[MOMX + 2 * (DIM > 2)] : 0.0, cm[ENERGY], one_l);
@@ -288,6 +300,55 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
       T const vr = cp[mP] * one_r;
       pol.template riemann<DIM, DIR, T>(eos, cm, cp, T(pm), T(pp), vl, vr, one_l, one_r, flux);
     } else {
+      if constexpr (ALP_FAST && sizeof(T) == 4) {
+        // FP32 form: the variations of the state and the physical flux projected
+        // as the two lanes of packed f32x2 arithmetic, the split fluxes'
+        // differences reconstructed with both sides as lanes; the left cell's
+        // flux (its characteristic values restored by R) added back in double
+        float2 x[5][NE];
+        double f0[NE], fa[NE], fb[NE];
+        phys_flux<DIM, DIR>(eos, cons[0], fa);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          phys_flux<DIM, DIR>(eos, cons[m + 1], fb);
+#pragma unroll
+          for (int l = 0; l < NE; ++l) {
+            x[m][l] = make_float2(float(cons[m + 1][l] - cons[m][l]), float(fb[l] - fa[l]));
+            fa[l] = fb[l];
+            if (m == C - 1) f0[l] = fb[l];
+          }
+        }
+        T ev_nl0, ev_lin, ev_nl1;
+        pol.template fs_eigenvalues<DIM, DIR, T>(eos, r, pt, pn, ev_nl0, ev_lin, ev_nl1);
+#pragma unroll
+        for (int n = 0; n < NE; ++n) {
+          T L[NE];
+          left_row<DIM, DIR, T>(n, r, L);
+          float const alpha = n == 0 ? ev_nl0 : (n == NE - 1 ? ev_nl1 : ev_lin);
+          float A[5], N[5];
+#pragma unroll
+          for (int m = 0; m < 5; ++m) {
+            float2 acc = make_float2(0.0f, 0.0f);
+            bool first = true;
+#pragma unroll
+            for (int q = 0; q < NE; ++q) {
+              int const l = sum_seq<DIM, DIR>(q);
+              if (!left_nonzero<DIM, DIR>(n, l)) continue;
+              acc = first ? mul2(x[m][l], dup2(L[l])) : fma2(x[m][l], dup2(L[l]), acc);
+              first = false;
+            }
+            A[m] = fmaf(alpha, acc.x, acc.y);
+            N[m] = fmaf(-alpha, acc.x, acc.y);
+          }
+          float2 const i = weno5_packed(make_float2(A[0], N[4]), make_float2(A[1], N[3]),
+                                        make_float2(A[2], N[2]), make_float2(A[3], N[1]), 1.0e-6f);
+          ch[0][n] = 0.5f * (i.x + (N[2] - i.y));
+        }
+        to_physical<DIM, DIR, T>(r, ch[0], flux);
+#pragma unroll
+        for (int f = 0; f < NE; ++f) fd[f] = f0[f] + double(flux[f]);
+        return valid;
+      }
       // Roe flux-vector splitting (flux_splitting_scheme.cpp:42-76, 185-315)
       double advd[W][NE];
 #pragma unroll
@@ -324,23 +385,6 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
         for (int m = 0; m < W; ++m) {
           T sp = T(0), sn = T(0);
           bool first = true;
-          if constexpr (DELTA && ALP_FAST) {
-            // state and flux projections as the two lanes of packed f32x2
-            // arithmetic: (L u, L f) += L[l] (du, df)
-            float2 acc = make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (int q = 0; q < NE; ++q) {
-              int const l = sum_seq<DIM, DIR>(q);
-              if (!left_nonzero<DIM, DIR>(n, l)) continue;
-              float2 const d = make_float2(float(cons[m][l] - cons[C][l]),
-                                           float(advd[m][l] - advd[C][l]));
-              acc = first ? mul2(d, dup2(L[l])) : fma2(d, dup2(L[l]), acc);
-              first = false;
-            }
-            pos[m] = fmaf(alpha, acc.x, acc.y);
-            neg[m] = fmaf(-alpha, acc.x, acc.y);
-            continue;
-          }
 #pragma unroll
           for (int q = 0; q < NE; ++q) {
             int const l = sum_seq<DIM, DIR>(q);
@@ -411,6 +455,27 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
     }
     if constexpr (sizeof(T) == 4) {
       // FP32 form: WENO5 of the increments against the left cell's primes
+      if constexpr (ALP_FAST) {
+        double pm[NE], pp[NE];
+#pragma unroll
+        for (int n = 0; n < NE; ++n) {
+          float G[5];
+#pragma unroll
+          for (int m = 0; m < 5; ++m) G[m] = float(prim[m + 1][n] - prim[m][n]);
+          float2 const i = weno5_packed(make_float2(G[0], G[4]), make_float2(G[1], G[3]),
+                                        dup2(G[2]), make_float2(G[3], G[1]), 1.0e-6f);
+          pm[n] = prim[C][n] + double(i.x);
+          pp[n] = prim[C + 1][n] - double(i.y);
+        }
+        if (!(pm[RHO] > DBL_EPSILON) || !(pp[RHO] > DBL_EPSILON)) valid = false;
+        if (!(pm[PRES] > -B) || !(pp[PRES] > -B)) valid = false;
+        hllc_flux_primes<DIM, DIR>(eos,
+                                   hllc_upwind_mixed(eos, pm[RHO], pp[RHO], pm[PRES], pp[PRES],
+                                                     pm[VELX + DIR], pp[VELX + DIR], inv(pm[RHO]),
+                                                     inv(pp[RHO])),
+                                   pm, pp, fd);
+        return valid;
+      }
       double pmd[NE], ppd[NE];
 #pragma unroll
       for (int n = 0; n < NE; ++n) {
@@ -461,19 +526,11 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
         // the upwind side's conservatives alone (hllc_upwind)
         if (!(pm[RHO] > DBL_EPSILON) || !(pp[RHO] > DBL_EPSILON)) valid = false;
         if (!(pm[PRES] > -B) || !(pp[PRES] > -B)) valid = false;
-        HllcUpwind const h = hllc_upwind(eos, pm[RHO], pp[RHO], pm[PRES], pp[PRES],
-                                         pm[VELX + DIR], pp[VELX + DIR], inv(pm[RHO]),
-                                         inv(pp[RHO]));
-        fd[MASS] = h.rho * h.k;
-        double q = 0.0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          double const v = h.right ? pp[VELX + d] : pm[VELX + d];
-          q = d == 0 ? v * v : fma(v, v, q);
-          fd[MOMX + d] = d == DIR ? fma(h.rho, h.g, h.p) : v * fd[MASS];
-        }
-        double const E = fma(0.5 * h.rho, q, (h.p + eos.gamma * eos.B) * inv(eos.gamma - 1.0));
-        fd[ENERGY] = fma(E, h.k, h.pe);
+        hllc_flux_primes<DIM, DIR>(eos,
+                                   hllc_upwind(eos, pm[RHO], pp[RHO], pm[PRES], pp[PRES],
+                                               pm[VELX + DIR], pp[VELX + DIR], inv(pm[RHO]),
+                                               inv(pp[RHO])),
+                                   pm, pp, fd);
         return valid;
       }
       // PrimeStatesToConservatives (prime_state_handler.h:195-275)

@@ -120,29 +120,11 @@ template <int DIM, typename T> __device__ __forceinline__ T dacms(T a, T b, T c)
   else return cms3(a, b, c);
 }
 
-// Sum of three squares, independent of the order of its terms as the
-// consistency-managed sum is. The fast build sorts them (the bit patterns of
-// non-negative floating-point values order like the values) and adds the two
-// smaller first: two additions and integer compares instead of seven
-// additions and four floating-point compares. The strict build and 1D/2D keep
-// DimensionAwareConsistencyManagedSum.
+// Sum of three squares: DimensionAwareConsistencyManagedSum in the strict build;
+// the fast build adds them in order.
 template <int DIM, typename T> __device__ __forceinline__ T sum_sq(T a, T b, T c) {
-  if constexpr (!ALP_FAST || DIM < 3) {
-    return dacms<DIM>(a, b, c);
-  } else if constexpr (sizeof(T) == 8) {
-    long long const ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-    long long const ic = __double_as_longlong(c);
-    long long const lo = min(ia, ib), hi = max(ia, ib);
-    long long const x0 = min(lo, ic), t = max(lo, ic);
-    long long const x1 = min(t, hi), x2 = max(t, hi);
-    return (__longlong_as_double(x0) + __longlong_as_double(x1)) + __longlong_as_double(x2);
-  } else {
-    int const ia = __float_as_int(a), ib = __float_as_int(b), ic = __float_as_int(c);
-    int const lo = min(ia, ib), hi = max(ia, ib);
-    int const x0 = min(lo, ic), t = max(lo, ic);
-    int const x1 = min(t, hi), x2 = max(t, hi);
-    return (__int_as_float(x0) + __int_as_float(x1)) + __int_as_float(x2);
-  }
+  if constexpr (!ALP_FAST || DIM < 3) return dacms<DIM>(a, b, c);
+  else return (a + b) + c;
 }
 
 // ---- stiffened gas (generic_stiffened_gas.h:40-102, stiffened_gas.cpp:62-149,
@@ -315,58 +297,43 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 // a - b, rounded once (a + (-1) b)
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, dup2(-1.0f), a); }
 
-// UpwindLeft and UpwindRight of one face, packed: P_k = (a[k], a[5-k]) for
-// k = 0 .. 4 of the six cells a[0..5] (i-2 .. i+3). Lane y runs the mirrored
-// stencil; both lanes end as P_2 + num / (6 den), with the indicators
-// 13/3 d_k^2 + e_k^2 (four times the reference's, eps likewise) and the ideal
-// weights as 1, 6, 3. The t_k are first multiplied by the power of two that
-// brings the largest into [1, 2) (exact: the scale is built from the exponent
-// bits), so the products stay inside the float range; a product that underflows
-// belongs to a weight below 2^-126 of the largest. One reciprocal per side (a
-// scaled denominator can be as small as the ratio of two smoothness terms, so
-// the product of two could underflow).
-__device__ __forceinline__ float2 weno5_packed(float2 P0, float2 P1, float2 P2, float2 P3,
-                                               float2 P4) {
-  float2 const ng1 = sub2(P0, P1), g2 = sub2(P2, P1), g3 = sub2(P3, P2), ng4 = sub2(P3, P4);
-  float2 const d1 = add2(g2, ng1), d2 = sub2(g3, g2), d3 = add2(ng4, g3);
-  float2 const e1 = fma2(dup2(3.0f), g2, ng1);
-  float2 const e2 = add2(g2, g3);
-  float2 const e3 = fma2(dup2(3.0f), g3, ng4);
-  float2 const c = dup2(13.0f / 3.0f), eps = dup2(4.0e-6f);
-  float2 const s1 = fma2(mul2(c, d1), d1, fma2(e1, e1, eps));
-  float2 const s2 = fma2(mul2(c, d2), d2, fma2(e2, e2, eps));
-  float2 const s3 = fma2(mul2(c, d3), d3, fma2(e3, e3, eps));
+// weno5_frac of both sides of a face as the lanes of packed arithmetic: lane x
+// from the first differences g1..g4 of the UpwindLeft stencil, lane y from those
+// of the mirrored UpwindRight stencil (reversed, sign kept). Returns the
+// increments num / (6 den). The t_k are first multiplied by the power of two
+// that brings the largest into [1, 2) (exact: the scale is built from the
+// exponent bits), so the products stay inside the float range; a product that
+// underflows belongs to a weight below 2^-126 of the largest. One reciprocal per
+// side (a scaled denominator can be as small as the ratio of two smoothness
+// terms, so the product of two could underflow).
+__device__ __forceinline__ float2 weno5_packed(float2 g1, float2 g2, float2 g3, float2 g4,
+                                               float eps) {
+  float2 const two = dup2(2.0f), c = dup2(4.0f / 3.0f), e = dup2(eps);
+  float2 const d1 = sub2(g2, g1), d2 = sub2(g3, g2), d3 = sub2(g4, g3);
+  float2 const a = add2(g2, d1), b = sub2(g3, d3);
+  float2 const s1 = fma2(g2, a, fma2(mul2(c, d1), d1, e));
+  float2 const s2 = fma2(g2, g3, fma2(mul2(c, d2), d2, e));
+  float2 const s3 = fma2(g3, b, fma2(mul2(c, d3), d3, e));
+  float2 const r1 = fma2(two, a, g2), r2 = fma2(two, g3, g2), r3 = fma2(two, g3, b);
   float2 const t1 = mul2(s1, s1), t2 = mul2(s2, s2), t3 = mul2(s3, s3);
-  float2 const r1 = fma2(dup2(2.0f), ng1, mul2(dup2(5.0f), g2));
-  float2 const r2 = fma2(dup2(2.0f), g3, g2);
-  float2 const r3 = fma2(dup2(4.0f), g3, ng4);
   // per lane: the power of two that brings the largest t_k into [1, 2)
   unsigned const ex = min((__float_as_uint(fmaxf(t1.x, fmaxf(t2.x, t3.x))) >> 23) & 0xffu, 253u);
   unsigned const ey = min((__float_as_uint(fmaxf(t1.y, fmaxf(t2.y, t3.y))) >> 23) & 0xffu, 253u);
   float2 const sc = make_float2(__uint_as_float((254u - ex) << 23), __uint_as_float((254u - ey) << 23));
   float2 const u1 = mul2(t1, sc), u2 = mul2(t2, sc), u3 = mul2(t3, sc);
-  float2 const b1 = mul2(u2, u3);
-  float2 const b2 = mul2(dup2(6.0f), mul2(u1, u3));
-  float2 const b3 = mul2(dup2(3.0f), mul2(u1, u2));
-  float2 const num = fma2(b3, r3, fma2(b2, r2, mul2(b1, r1)));
-  float2 const q = mul2(dup2(6.0f), add2(add2(b1, b2), b3));
-  return fma2(num, make_float2(inv(q.x), inv(q.y)), P2);
+  float2 const y = mul2(dup2(3.0f), u1), z = add2(u3, u3), p = mul2(u2, u3);
+  float2 const num = fma2(y, fma2(z, r2, mul2(u2, r3)), mul2(p, r1));
+  float2 const q = mul2(dup2(6.0f), fma2(y, add2(z, u2), p));
+  return mul2(num, make_float2(inv(q.x), inv(q.y)));
 }
 
 // UpwindLeft and UpwindRight of one face from the same six cells a[0..5]
-// (i-2..i+3): weno5_increments (fast build, double) or the two sides as the
-// lanes of packed f32x2 arithmetic (float).
+// (i-2..i+3).
 template <typename T>
 __device__ __forceinline__ void weno5_pair(T const (&a)[6], T &left, T &right) {
   if constexpr (!ALP_FAST) {
     left = weno5_left(a);
     right = weno5_right(a);
-  } else if constexpr (sizeof(T) == 4) {
-    float2 const r = weno5_packed(make_float2(a[0], a[5]), make_float2(a[1], a[4]),
-                                  make_float2(a[2], a[3]), make_float2(a[3], a[2]),
-                                  make_float2(a[4], a[1]));
-    left = r.x;
-    right = r.y;
   } else {
     double const G[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], a[5] - a[4]};
     double l, r;
@@ -383,13 +350,6 @@ __device__ __forceinline__ void weno5_two(T const (&a)[6], T const (&b)[6], T &l
   if constexpr (!ALP_FAST) {
     left = weno5_left(a);
     right = weno5_right(b);
-  } else if constexpr (sizeof(T) == 4) {
-    // lane y: b mirrored
-    float2 const r = weno5_packed(make_float2(a[0], b[5]), make_float2(a[1], b[4]),
-                                  make_float2(a[2], b[3]), make_float2(a[3], b[2]),
-                                  make_float2(a[4], b[1]));
-    left = r.x;
-    right = r.y;
   } else {
     double const A[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], 0.0};
     double const B[5] = {0.0, b[2] - b[1], b[3] - b[2], b[4] - b[3], b[5] - b[4]};
@@ -831,6 +791,40 @@ __device__ __forceinline__ HllcUpwind hllc_upwind(Eos const &e, double rl, doubl
   return h;
 }
 
+// Flux of the upwind star state from its side's conserved state.
+template <int DIM, int DIR>
+__device__ __forceinline__ void hllc_flux(HllcUpwind const &h, double const (&cl)[DIM + 2],
+                                          double const (&cr)[DIM + 2], double (&flux)[DIM + 2]) {
+  constexpr int mP = MOMX + DIR;
+  flux[MASS] = h.rho * h.k;
+  flux[mP] = fma(h.rho, h.g, h.p);
+  flux[ENERGY] = fma(h.right ? cr[ENERGY] : cl[ENERGY], h.k, h.pe);
+#pragma unroll
+  for (int d = 0; d < DIM - 1; ++d) {
+    int const mm = MOMX + (d == 0 ? Minor<DIR>::m1 : Minor<DIR>::m2);
+    flux[mm] = (h.right ? cr[mm] : cl[mm]) * h.k;
+  }
+}
+
+// Its flux from prime states (Density, Pressure, VelocityX..): the upwind side's
+// conserved quantities alone.
+template <int DIM, int DIR>
+__device__ __forceinline__ void hllc_flux_primes(Eos const &e, HllcUpwind const &h,
+                                                 double const (&pm)[DIM + 2],
+                                                 double const (&pp)[DIM + 2],
+                                                 double (&flux)[DIM + 2]) {
+  flux[MASS] = h.rho * h.k;
+  double q = 0.0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    double const v = h.right ? pp[VELX + d] : pm[VELX + d];
+    q = d == 0 ? v * v : fma(v, v, q);
+    flux[MOMX + d] = d == DIR ? fma(h.rho, h.g, h.p) : v * flux[MASS];
+  }
+  double const E = fma(0.5 * h.rho, q, (h.p + e.gamma * e.B) * inv(e.gamma - 1.0));
+  flux[ENERGY] = fma(E, h.k, h.pe);
+}
+
 // CalculateSignalSpeed, Einfeldt (hll_signal_speed_calculator.h:77-101) and
 // HllcRiemannSolver::SolveRiemannProblemImplementation (hllc_riemann_solver.h:52-198)
 // one_rl, one_rr: 1/density of the two states as returned by inv()
@@ -841,16 +835,9 @@ __device__ __forceinline__ void hllc(Eos const &e, T const (&cl)[DIM + 2], T con
   constexpr int NE = DIM + 2;
   constexpr int mP = MOMX + DIR;
   if constexpr (ALP_FAST && sizeof(T) == 8) {
-    HllcUpwind const h = hllc_upwind(e, cl[MASS], cr[MASS], pres_l, pres_r, vel_l, vel_r, one_rl,
-                                     one_rr);
-    flux[MASS] = h.rho * h.k;
-    flux[mP] = fma(h.rho, h.g, h.p);
-    flux[ENERGY] = fma(h.right ? cr[ENERGY] : cl[ENERGY], h.k, h.pe);
-#pragma unroll
-    for (int d = 0; d < DIM - 1; ++d) {
-      int const mm = MOMX + (d == 0 ? Minor<DIR>::m1 : Minor<DIR>::m2);
-      flux[mm] = (h.right ? cr[mm] : cl[mm]) * h.k;
-    }
+    hllc_flux<DIM, DIR>(hllc_upwind(e, cl[MASS], cr[MASS], pres_l, pres_r, vel_l, vel_r, one_rl,
+                                    one_rr),
+                        cl, cr, flux);
     return;
   }
   T const c_l = eos_speed_of_sound<T>(e, cl[MASS], pres_l, one_rl);
@@ -909,7 +896,41 @@ __device__ __forceinline__ void hllc(Eos const &e, T const (&cl)[DIM + 2], T con
   (void)NE;
 }
 
-// HLLC for the FP32-flux form (same approximate Riemann solver as hllc():
+// hllc_upwind of the FP32-flux form: wave speeds, the contact speed and the
+// increments against the upwind state's physical flux in float, that flux and
+// the sums in double. Uses chi - 1 = (S* - v) / (S - S*), so no increment is
+// formed by cancellation.
+__device__ __forceinline__ HllcUpwind hllc_upwind_mixed(Eos const &e, double rl, double rr,
+                                                        double pl, double pr, double vl, double vr,
+                                                        double one_l, double one_r) {
+  float const ccl = float(eos_cc(e, rl, pl, one_l)), ccr = float(eos_cc(e, rr, pr, one_r));
+  float const frl = float(rl), frr = float(rr), ul = float(vl), ur = float(vr);
+  float const srl = tsqrt(frl), srr = tsqrt(frr);
+  float const one = inv(srl + srr);
+  float const wl = srl * one, wr = srr * one;
+  float const du = float(vl - vr);
+  float const u = fmaf(wl, du, ur);
+  float const ce = tsqrt(fmaf(0.5f * (wl * wr), du * du, fmaf(wl, ccl - ccr, ccr)));
+  float const sl = dmin(u - ce, ul - tsqrt(ccl)), sr = dmax(u + ce, ur + tsqrt(ccr));
+  float const al = frl * (sl - ul), ar = frr * (sr - ur);
+  float const ss = fmaf(ul, al, fmaf(-ur, ar, float(pr - pl))) * inv(al - ar);
+  HllcUpwind h;
+  h.right = ss < 0.0f;
+  h.rho = h.right ? rr : rl;
+  h.p = h.right ? pr : pl;
+  double const v = h.right ? vr : vl;
+  float const fu = h.right ? ur : ul, s = h.right ? sr : sl;
+  float const sc = h.right ? dmax(sr, 0.0f) : dmin(sl, 0.0f);
+  float const dss = ss - fu;
+  float const dchi = dss * inv(s - ss);
+  h.k = v + double(sc * dchi);
+  h.g = fma(v, v, double(sc * fmaf(dchi, ss, dss)));
+  h.pe = fma(v, h.p, double((sc * ((1.0f + dchi) * dss)) *
+                            fmaf(h.right ? frr : frl, ss, float(h.p) * inv(sc - fu))));
+  return h;
+}
+
+// HLLC for the strict build's FP32-flux form (same approximate Riemann solver as hllc():
 // Einfeldt speeds, Toro star states, the reference's clamped-speed energy
 // term). Wave speeds, the contact speed and the star-state increments
 // q* - q are computed in float; the physical fluxes F(q) that carry the mean
@@ -938,35 +959,6 @@ __device__ __forceinline__ void hllc_mixed(Eos const &e, double const (&cl)[DIM 
   float const s_star = __fdividef(dpr + (rl * ul * (sls - ul) - rr * ur * (srs - ur)),
                                   rl * (sls - ul) - rr * (srs - ur));
   float const sl = dmin(sls, 0.0f), sr = dmax(srs, 0.0f);
-  if constexpr (ALP_FAST) {
-    // the upwind star flux alone (as in hllc())
-    bool const rs = s_star < 0.0f;
-    float const rho = rs ? rr : rl, u = rs ? ur : ul;
-    float const s = rs ? srs : sls, sc = rs ? sr : sl;
-    double const p = rs ? pres_r : pres_l, v = rs ? vel_r : vel_l;
-    double const one_r = rs ? one_rr : one_rl;
-    double const mp = rs ? cr[mP] : cl[mP], E = rs ? cr[ENERGY] : cl[ENERGY];
-    float const dchi = __fdividef(s_star - u, s - s_star);  // chi - 1
-    float dq[DIM + 2];
-    double f[DIM + 2];
-    dq[MASS] = rho * dchi;
-    dq[mP] = rho * ((s_star - u) + dchi * s_star);
-    dq[ENERGY] = float(E) * dchi + rho * (1.0f + dchi) * (s_star - u) *
-                                       (s_star + __fdividef(float(p), rho * (sc - u)));
-    f[MASS] = mp;
-    f[mP] = mp * mp * one_r + p;
-    f[ENERGY] = v * (E + p);
-#pragma unroll
-    for (int d = 0; d < DIM - 1; ++d) {
-      int const mm = MOMX + (d == 0 ? Minor<DIR>::m1 : Minor<DIR>::m2);
-      double const q = rs ? cr[mm] : cl[mm];
-      dq[mm] = dchi * float(q);
-      f[mm] = v * q;
-    }
-#pragma unroll
-    for (int n = 0; n < DIM + 2; ++n) flux[n] = f[n] + double(sc * dq[n]);
-    return;
-  }
   float const dchi_l = __fdividef(s_star - ul, sls - s_star);  // chi_l - 1
   float const dchi_r = __fdividef(s_star - ur, srs - s_star);
   float const chi_l = 1.0f + dchi_l, chi_r = 1.0f + dchi_r;
