@@ -21,8 +21,9 @@ PROBE_LIB = os.path.join(HERE, "libalpaca_b200_probe.so")
 # its own, as in the reference's x86-64 build. Tests use it to show that the
 # CUDA arithmetic follows the reference's operation order bit for bit.
 STRICT_LIB = os.path.join(HERE, "libalpaca_b200_strict.so")
-SOURCES = ["kernels.cu", "face_flux.cu", "pencil.cu", "sweep.cu", "ext_first_order.cu",
-           "ext_weno3.cu", "ext_weno5.cu", "ext_weno5z.cu", "ext_teno5.cu", "ext_weno7.cu", "capi.cu", "server.cu", "levels.cu", "static_scratch.cu", "ic_expr.cu",
+SOURCES = ["kernels.cu", "face_flux.cu", "pencil.cu", "sweep.cu", "small.cu",
+           "ext_first_order.cu", "ext_weno3.cu", "ext_weno5.cu", "ext_weno5z.cu", "ext_teno5.cu",
+           "ext_weno7.cu", "capi.cu", "server.cu", "levels.cu", "static_scratch.cu", "ic_expr.cu",
            "elastic.cu",
            "tile_step.cu", "tile_step_fvchar.cu", "tile_step_fvprim.cu", "tile_step_fsroe.cu"]
 PROBE_SOURCES = ["probe.cu"]

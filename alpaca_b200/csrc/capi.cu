@@ -637,6 +637,7 @@ int alp_engine_step(alp_engine *e, int n) {
   // profiler ranges (no cost unless a tool is attached): one per call, one per capture
   nvtx3::scoped_range range{"alp_engine_step"};
   if (e->path == 3) return e->run_tiles(n);
+  if (e->small_steps()) return e->record_step(false, n);
   if (!e->use_graph) {
     for (int i = 0; i < n; ++i)
       if (int rc = e->record_step()) return rc;
@@ -895,13 +896,15 @@ int alp_engine_launches_per_step(alp_engine *e) {
   // fluxes + stage update, per batch on the overlapped path), commit; the tile
   // path launches signal speed, dt and one persistent kernel per call
   if (e->path == 3) return 3;
+  if (e->small_steps()) return 1;
   int const batches = e->path == 2 ? std::min(alp_engine::kMaxBatches, std::max(1, e->nwork / 64)) : 1;
   return 2 + (e->rk2 ? 2 : 3) * (e->path == 0 ? e->dim : 2 * batches) + 1;
 }
 
 int alp_engine_launches(alp_engine *e, int n) {
   if (!e || n <= 0 || e->nwork == 0) return 0;
-  return e->path == 3 ? 3 : n * alp_engine_launches_per_step(e);
+  if (e->path == 3) return 3;
+  return e->small_steps() ? small_launches(n) : n * alp_engine_launches_per_step(e);
 }
 
 }  // extern "C"

@@ -121,19 +121,33 @@ struct alp_engine {
   long long dstride() const { return (long long)ne * faces; }
   long long stride() const { return dstride() * dim; }
 
+  // Whether the face-flux path runs whole steps in one launch (small.cu).
+  bool small_steps() const {
+    return path == 1 && opt.is_default() && alp::small_pays(dim, nwork);
+  }
+
   // dt, then per stage the fluxes and the stage update: A -> B, (B, A) -> C,
   // (C, A) -> A. trial: the last stage writes B instead of A and the step is
   // not committed, so the case state is left as it was (autotuning).
-  int record_step(bool trial = false) {
+  // n > 1: small work lists only (small_steps).
+  int record_step(bool trial = false, int n = 1) {
     Launch L{dim, scheme, precision, U, work, nwork, meta, BlockMeta{}, stream};
     L.opt = opt;
-    ALP_CUDA(launch_signal_speed(L, cases, nullptr));
-    ALP_CUDA(launch_dt_finalize(cases, max_cases, stream));
+    bool const small = small_steps();
+    if (!small) {
+      ALP_CUDA(launch_signal_speed(L, cases, nullptr));
+      ALP_CUDA(launch_dt_finalize(cases, max_cases, stream));
+    }
     // RK3: A -> B, (B, A) -> C, (C, A) -> A; RK2: A -> B, (B, A) -> A (trial: C)
     double *in[3] = {U, UB, UC};
     double *out[3] = {UB, UC, trial ? UB : U};
     if (rk2) out[1] = trial ? UC : U;
     int const nst = rk2 ? 2 : 3, s0 = rk2 ? 3 : 0;
+    if (small) {
+      ALP_CUDA(alp::launch_small_steps(L, in, out, F, stride(), dstride(), nbr26, cases, max_cases,
+                                       nst, s0, n, !trial));
+      return ALP_OK;
+    }
     bool const glf_due = scheme == alp::FS_ROE && opt.splitting == alp::FSP_GLF;
     for (int s = 0; s < nst; ++s) {
       Launch Ls = L;

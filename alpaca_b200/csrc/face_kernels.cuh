@@ -82,7 +82,7 @@ __device__ __forceinline__ void write_flux(double *__restrict__ F, int item, lon
 // GATHER: cells outside the interior along DIR come from the neighbour blocks'
 // interiors (nbr26; zero gradient at domain faces) instead of the block's own
 // halo cells, so no halo copy is needed between stages.
-template <int DIM, int DIR, bool GATHER>
+template <int DIM, int DIR, int GATHER>
 __device__ __forceinline__ double const *stencil_cell(double const *__restrict__ U,
                                                       double const *blk, int c, int cell0,
                                                       int nlo, int nhi) {
@@ -109,33 +109,36 @@ __device__ __forceinline__ int line_origin(int p1, int p2) {
   return G::cell(c[0], c[1], c[2]);
 }
 
-template <int DIM, int DIR>
+// GATHER of the loads below: 0 the block's own halo cells, 1 the neighbours'
+// interiors, 2 the same through L2 (cells written earlier in the same launch).
+template <int DIM, int GATHER>
 __device__ __forceinline__ void load_cell(double const *src, double (&dst)[DIM + 2]) {
 #pragma unroll
-  for (int f = 0; f < DIM + 2; ++f) dst[f] = __ldg(src + f * Geo<DIM>::CELLS);
+  for (int f = 0; f < DIM + 2; ++f)
+    dst[f] = GATHER == 2 ? __ldcg(src + f * Geo<DIM>::CELLS) : __ldg(src + f * Geo<DIM>::CELLS);
 }
 
 // Cell c of a stencil line (stencil_cell), with symmetry walls: a neighbour
 // entry of -2 across the block face mirrors the line about the wall and negates
 // the momentum normal to it (symmetry_boundary_condition.h:60-113, 148-217;
 // boundary_constants.h:35-46, 167-209); -1 is zero gradient.
-template <int DIM, int DIR, bool GATHER>
+template <int DIM, int DIR, int GATHER>
 __device__ __forceinline__ void stencil_load(double const *__restrict__ U, double const *blk,
                                              int c, int cell0, int nlo, int nhi,
                                              double (&dst)[DIM + 2]) {
   constexpr int step = DIR == 0 ? Geo<DIM>::TCY * Geo<DIM>::TCZ : (DIR == 1 ? Geo<DIM>::TCZ : 1);
   if (GATHER && ((c < HS && nlo == -2) || (c >= HS + IC && nhi == -2))) {
     int const m = c < HS ? 2 * HS - 1 - c : 2 * (HS + IC) - 1 - c;
-    load_cell<DIM, DIR>(blk + cell0 + m * step, dst);
+    load_cell<DIM, GATHER>(blk + cell0 + m * step, dst);
     dst[MOMX + DIR] = -1.0 * dst[MOMX + DIR];
     return;
   }
-  load_cell<DIM, DIR>(stencil_cell<DIM, DIR, GATHER>(U, blk, c, cell0, nlo, nhi), dst);
+  load_cell<DIM, GATHER>(stencil_cell<DIM, DIR, GATHER>(U, blk, c, cell0, nlo, nhi), dst);
 }
 
 // Flux of the face (a; p1, p2) of direction DIR of the block in `slot`; false
 // for a face the reference skips.
-template <int DIM, int DIR, int SCHEME, typename T, bool GATHER, typename P = DefaultPolicy,
+template <int DIM, int DIR, int SCHEME, typename T, int GATHER, typename P = DefaultPolicy,
           int W = 6>
 __device__ __forceinline__ bool face_value(double const *__restrict__ U,
                                            int const *__restrict__ nbr26, int slot, int a, int p1,
@@ -175,7 +178,7 @@ __device__ __forceinline__ bool face_value(double const *__restrict__ U,
 }
 
 // Flux of the face with thread index t of direction DIR of the block in `slot`.
-template <int DIM, int DIR, int SCHEME, typename T, bool ACCUM, bool GATHER,
+template <int DIM, int DIR, int SCHEME, typename T, bool ACCUM, int GATHER,
           typename P = DefaultPolicy, int W = 6>
 __device__ __forceinline__ void face_flux(double const *__restrict__ U,
                                           int const *__restrict__ nbr26, int slot, int item,

@@ -102,6 +102,17 @@ cudaError_t launch_sweep_update(Launch const &L, double const *U0, double *Uout,
                                 long long flux_item_stride, long long dir_stride,
                                 int const *nbr26, CaseState const *cases, int stage);
 
+// n whole steps of a small 1D or 2D work list (default schemes) in one launch
+// per 256 steps: signal speed, dt, nst stages of in[s] -> out[s] (stage table
+// rows from s0) and, with commit, t and the step counts; L.U is the state at the
+// step's start. small_pays: whether nwork blocks step faster that way.
+bool small_pays(int dim, int nwork);
+int small_launches(int n);
+cudaError_t launch_small_steps(Launch const &L, double *const in[3], double *const out[3],
+                               double *F, long long flux_item_stride, long long dir_stride,
+                               int const *nbr26, CaseState *cases, int ncases, int nst, int s0,
+                               int n, bool commit);
+
 // One SSP-RK3 stage of every work item by pencil sweeps (engine fast path):
 // the faces of each line of cells along x, then y, then z, with the
 // per-cell flux differences accumulated in R ([slot][NE][interior cells]) and

@@ -52,18 +52,25 @@ __device__ __forceinline__ double flux_divergence(double fx_lo, double fx_hi, do
   return dacms<DIM>(dx, dy, dz) * one_cell_size;
 }
 
+// A load through L2 (CG: values written earlier in the same launch) or as usual.
+template <bool CG> __device__ __forceinline__ double ld(double const *p) {
+  return CG ? __ldcg(p) : *p;
+}
+
 // Flux divergence of interior cell (i, j, k) of one field from the reference
 // flux arrays of the three directions (Fx, Fy, Fz at the field's offset).
-template <int DIM>
+template <int DIM, bool CG = false>
 __device__ __forceinline__ double divergence(double const *Fx, double const *Fy,
                                              double const *Fz, int i, int j, int k,
                                              double one_cell_size) {
   using G = Geo<DIM>;
-  return flux_divergence<DIM>(Fx[G::face(i, j + 1, k + 1)], Fx[G::face(i + 1, j + 1, k + 1)],
-                              DIM > 1 ? Fy[G::face(i + 1, j, k + 1)] : 0.0,
-                              DIM > 1 ? Fy[G::face(i + 1, j + 1, k + 1)] : 0.0,
-                              DIM > 2 ? Fz[G::face(i + 1, j + 1, k)] : 0.0,
-                              DIM > 2 ? Fz[G::face(i + 1, j + 1, k + 1)] : 0.0, one_cell_size);
+  return flux_divergence<DIM>(ld<CG>(Fx + G::face(i, j + 1, k + 1)),
+                              ld<CG>(Fx + G::face(i + 1, j + 1, k + 1)),
+                              DIM > 1 ? ld<CG>(Fy + G::face(i + 1, j, k + 1)) : 0.0,
+                              DIM > 1 ? ld<CG>(Fy + G::face(i + 1, j + 1, k + 1)) : 0.0,
+                              DIM > 2 ? ld<CG>(Fz + G::face(i + 1, j + 1, k)) : 0.0,
+                              DIM > 2 ? ld<CG>(Fz + G::face(i + 1, j + 1, k + 1)) : 0.0,
+                              one_cell_size);
 }
 
 // Interior cell (i, j, k) of thread t of a block's 16^DIM cells (z fastest).
@@ -87,7 +94,7 @@ __host__ __device__ __forceinline__ void interior_coords(int t, int &i, int &j, 
 // Stage update of interior cell t of the block in `slot`, every field: the flux
 // divergence from the block's face-flux arrays Fb (directions dstride apart)
 // and the RK stage into Uout. Every stage update computes it this way.
-template <int DIM>
+template <int DIM, bool CG = false>
 __device__ __forceinline__ void stage_update_cell(double const *Uin, double const *U0, double *Uout,
                                                   double const *Fb, long long dstride, int slot,
                                                   int t, double one_cell_size, RkStage const &rk) {
@@ -102,10 +109,11 @@ __device__ __forceinline__ void stage_update_cell(double const *Uin, double cons
 #pragma unroll
   for (int f = 0; f < G::NE; ++f) {
     double const *fx = Fb + f * G::FACES;
-    rhs[f] = 0.0 + divergence<DIM>(fx, fx + dstride, fx + 2 * dstride, i, j, k, one_cell_size);
+    rhs[f] =
+        0.0 + divergence<DIM, CG>(fx, fx + dstride, fx + 2 * dstride, i, j, k, one_cell_size);
     size_t const x = base + (size_t)f * G::CELLS;
-    u[f] = Uin[x];
-    u0[f] = rk.first ? 0.0 : U0[x];
+    u[f] = ld<CG>(Uin + x);
+    u0[f] = rk.first ? 0.0 : ld<CG>(U0 + x);
   }
 #pragma unroll
   for (int f = 0; f < G::NE; ++f)
