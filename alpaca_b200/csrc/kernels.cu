@@ -90,12 +90,22 @@ rk_stage_rhs_kernel(double *__restrict__ U, double *__restrict__ U0,
   interior_coords<DIM>(t, i, j, k);
   int const c = G::cell(i + G::fic(0), j + G::fic(1), k + G::fic(2));
   RkStage const rk = rk_stage(stage, dt);
+  size_t const base = (size_t)slot * G::BLOCK_DOUBLES + c;
+  // every load before the first store (the buffers may alias, as far as the
+  // compiler knows)
+  double u[G::NE], u0[G::NE], r[G::NE];
 #pragma unroll
   for (int f = 0; f < G::NE; ++f) {
-    size_t const x = (size_t)slot * G::BLOCK_DOUBLES + (size_t)f * G::CELLS + c;
-    double const u = U[x];
-    if (stage == 0) U0[x] = u;
-    U[x] = rk_apply(rk, u, rk.first ? 0.0 : U0[x], rhs[x]);
+    size_t const x = base + (size_t)f * G::CELLS;
+    u[f] = U[x];
+    u0[f] = rk.first ? 0.0 : U0[x];
+    r[f] = rhs[x];
+  }
+#pragma unroll
+  for (int f = 0; f < G::NE; ++f) {
+    size_t const x = base + (size_t)f * G::CELLS;
+    if (stage == 0) U0[x] = u[f];
+    U[x] = rk_apply(rk, u[f], u0[f], r[f]);
   }
 }
 
