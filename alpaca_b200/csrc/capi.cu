@@ -460,12 +460,15 @@ int engine_create(int dim, const alp_scheme *scheme, int capacity_blocks, int ma
     if (ok && (cudaGetDevice(&dev) != cudaSuccess ||
                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
       ok = false;
-    for (int v = 0; ok && v < alp::kTileVariants; ++v) {
-      if (alp::tile_info(sid, v, prec, &e->tinfo[v]) != cudaSuccess || e->tinfo[v].ctas_per_sm < 1)
-        ok = false;
-      else
-        e->tgrid[v] = e->tinfo[v].ctas_per_sm * sms;
-    }
+    for (int v = 0; ok && v < alp::kTileVariants; ++v)
+      for (int h = 0; ok && h < 3; ++h) {
+        alp::TileKernelInfo &k = e->tinfo[v][h];
+        if (alp::tile_info(sid, v, 16 >> h, prec, &k) != cudaSuccess || k.ctas_per_sm < 1 ||
+            (h && k.ctas_per_sm != e->tinfo[v][0].ctas_per_sm))
+          ok = false;
+        else
+          e->tgrid[v] = k.ctas_per_sm * sms;
+      }
     cudaGetLastError();  // a refused attribute or query leaves the face-flux path
     if (ok) {
       alp::TileArgs &a = e->targs;

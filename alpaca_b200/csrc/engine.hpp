@@ -90,8 +90,12 @@ struct alp_engine {
   bool tile_ok = false;       // 3D, default schemes, descriptors encoded
   int tile_variant = 0;       // index into alp::kTileWarps
   alp::TileArgs targs{};      // TMA descriptors and device pointers (nsteps set per launch)
-  alp::TileKernelInfo tinfo[alp::kTileVariants] = {};
+  alp::TileKernelInfo tinfo[alp::kTileVariants][3] = {};  // 1, 2, 4 items per block
   int tgrid[alp::kTileVariants] = {};
+  // the instantiation for the current work list
+  alp::TileKernelInfo const &tile_kernel() const {
+    return tinfo[tile_variant][alp::tile_parts(nwork, tgrid[tile_variant]) / 2];
+  }
   int *tsync = nullptr;       // [2 + capacity + 2 max_cases]: next item, error, block flags,
                               // dt flags, last-stage counts
   int *torder = nullptr;      // [3][capacity] block slots per stage, in readiness order
@@ -190,7 +194,7 @@ struct alp_engine {
     a.nsteps = n;
     a.trial = trial ? 1 : 0;
     // one CTA per SM and kernel variant; CTAs that find no item left return
-    ALP_CUDA(alp::tile_launch(a, tinfo[tile_variant], tgrid[tile_variant], stream));
+    ALP_CUDA(alp::tile_launch(a, tile_kernel(), tgrid[tile_variant], stream));
     return ALP_OK;
   }
 
@@ -226,7 +230,7 @@ struct alp_engine {
         cudaKernelNodeParams kp;
         if (cudaGraphNodeGetType(nd, &ty) == cudaSuccess && ty == cudaGraphNodeTypeKernel &&
             cudaGraphKernelNodeGetParams(nd, &kp) == cudaSuccess &&
-            kp.func == tinfo[tile_variant].fn)
+            kp.func == tile_kernel().fn)
           tile_node = nd;
       }
       cudaError_t const ie = cudaGraphInstantiate(&graph, g, 0);
@@ -245,10 +249,11 @@ struct alp_engine {
       a.trial = 0;
       void *args[] = {&a};
       cudaKernelNodeParams kp{};
-      kp.func = const_cast<void *>(tinfo[tile_variant].fn);
+      alp::TileKernelInfo const &tk = tile_kernel();
+      kp.func = const_cast<void *>(tk.fn);
       kp.gridDim = dim3(tgrid[tile_variant]);
-      kp.blockDim = dim3(tinfo[tile_variant].threads);
-      kp.sharedMemBytes = (unsigned)tinfo[tile_variant].smem;
+      kp.blockDim = dim3(tk.threads);
+      kp.sharedMemBytes = (unsigned)tk.smem;
       kp.kernelParams = args;
       kp.extra = nullptr;
       ALP_CUDA(cudaGraphExecKernelNodeSetParams(graph, tile_node, &kp));

@@ -23,9 +23,9 @@ struct TileArgs {
   CaseState *cases;
   int *ctrl;             // [0] next item; [1] error bits: 1 dependency, 2 load, 4 dt,
                          // 8 task-order wait ran out (not reset by the launches)
-  int *done;             // [slots] last finished (step, stage) + 1 of each block
+  int *done;             // [slots] finished items of each block
   int *dtflag;           // [cases] 1 + the step whose dt is ready
-  int *cnt;              // [cases] blocks of the case that finished a last stage
+  int *cnt;              // [cases] items of the case that finished a last stage
   int const *case_nb;    // [cases] blocks of each case in the work list
 };
 
@@ -42,11 +42,13 @@ constexpr int kTileVariants = 2;
 constexpr int kTileWarps[kTileVariants] = {16, 12};
 
 template <int SCHEME>
-cudaError_t tile_kernel_info(int variant, int precision, TileKernelInfo *out);
+cudaError_t tile_kernel_info(int variant, int planes, int precision, TileKernelInfo *out);
 
-// Shared-memory limit and launch shape of the kernel for a scheme id, variant
-// and precision.
-cudaError_t tile_info(int scheme, int variant, int precision, TileKernelInfo *out);
+// Shared-memory limit and launch shape of the kernel for a scheme id, variant,
+// x-planes per item (16, 8 or 4) and precision.
+cudaError_t tile_info(int scheme, int variant, int planes, int precision, TileKernelInfo *out);
+// Items per block (1, 2 or 4) with which nwork blocks step fastest on `ctas` CTAs.
+int tile_parts(int nwork, int ctas);
 // TMA descriptors of the three block pools (reference layout, `capacity`
 // blocks each) into a; false with a reason when the driver cannot encode them.
 bool tile_encode(TileArgs &a, double *const pools[3], int capacity, std::string &why);

@@ -1,23 +1,26 @@
 // Index plan of the fused tile-stage kernel (tile_step.cuh), as host and
 // device functions so that tests can replay it on the CPU.
 //
-// One work item is one SSP-RK3 (or TVD-RK2) stage of one 3D block. The block's
-// cells are walked in x-planes. Stencils are read from shared memory:
+// One work item is one SSP-RK3 (or TVD-RK2) stage of the x-planes x0 .. x0 +
+// NX - 1 of one 3D block: all 16, or a half or a quarter (NX = 8, 4) when the
+// blocks alone would leave SMs idle. Planes and faces are numbered from x0 (0 ..
+// NX - 1 below); planes beyond a part's inner ends are the block's own. The
+// item's cells are walked in x-planes. Stencils are read from shared memory:
 //   * a ring of RING x-planes (16 x 16 cells, all five conserved fields) of the
-//     stage input: planes -3 .. 18 in interior numbering, the six outside the
-//     block taken from the x neighbours, none at walls (the readers map those
+//     stage input: planes -3 .. NX + 2, those outside the block taken from the
+//     x neighbours, none at walls (the readers map those
 //     cells onto the block, stencil_src);
 //   * per plane, the three rows beyond each y face and the (aligned, four wide)
 //     columns beyond each z face, from the y / z neighbours.
 // The item is a stream of warp tasks, taken by the CTA's warps in order:
 //   X0              x face 0 (8 tasks of 32 faces)
-//   for g = 0 .. 15:
+//   for g = 0 .. NX - 1:
 //     U(g - LAG)    flux divergence and stage update of plane g - LAG (8 tasks
 //                   of 32 cells), for g >= LAG
 //     FX(g)         x face g + 1 (8 tasks)
 //     FY(g), FZ(g)  the 17 x 16 y faces and 16 x 17 z faces of plane g (9 tasks
 //                   each, the last one half full)
-//   U(16 - LAG) .. U(15)
+//   U(NX - LAG) .. U(NX - 1)
 // A plane's update trails its faces by LAG planes, so that the fluxes it reads
 // were computed a whole plane of tasks earlier, and the flux buffers it frees
 // are next written a plane of tasks later. Every task waits only for tasks
@@ -68,13 +71,14 @@ struct Src {
 // Written with selects only: the lanes of a warp hold faces at different
 // positions, and a branch here would split the warp for the whole face
 // computation that follows.
-__host__ __device__ inline Src stencil_src(int c, int nlo, int nhi) {
-  bool const lo = c < 0, out = lo || c >= IC;
+// ncell: the cells along the direction (IC; along x the item's planes).
+__host__ __device__ inline Src stencil_src(int c, int nlo, int nhi, int ncell = IC) {
+  bool const lo = c < 0, out = lo || c >= ncell;
   int const n = lo ? nlo : nhi;
   bool const wall = out && n < 0;
   bool const sym = wall && n == -2;
-  int const mirror = lo ? -1 - c : 2 * IC - 1 - c;
-  int const clamp = lo ? 0 : IC - 1;
+  int const mirror = lo ? -1 - c : 2 * ncell - 1 - c;
+  int const clamp = lo ? 0 : ncell - 1;
   int const index = !wall ? c : (sym ? mirror : clamp);
   return Src{index, !out || wall, sym};
 }
@@ -96,7 +100,10 @@ constexpr int UT = PLANE / 32;                  // of one plane's stage update (
 constexpr int FT = XT + 2 * YT;                  // face tasks of one plane (26)
 constexpr int ITER = FT + UT;                     // tasks of one plane g >= LAG (34)
 constexpr int LAG = 2;                            // planes between faces and update
-constexpr int STREAM = XT + LAG * FT + (IC - LAG) * ITER + LAG * UT;  // 552
+template <int NX> __host__ __device__ constexpr int stream_length() {
+  return XT + LAG * FT + (NX - LAG) * ITER + LAG * UT;
+}
+constexpr int STREAM = stream_length<IC>();  // 552 (280 and 144 of a half and a quarter)
 
 struct Task {
   int type;  // TaskType
@@ -109,17 +116,17 @@ __host__ __device__ inline Task face_task(int g, int r) {
   if (r < XT + YT) return Task{T_FY, g, r - XT};
   return Task{T_FZ, g, r - XT - YT};
 }
-__host__ __device__ inline Task decode(int pos) {
+template <int NX = IC> __host__ __device__ inline Task decode(int pos) {
   if (pos < XT) return Task{T_FX, 0, pos};
   pos -= XT;
   if (pos < LAG * FT) return face_task(pos / FT, pos % FT);
   pos -= LAG * FT;
-  if (pos < (IC - LAG) * ITER) {
+  if (pos < (NX - LAG) * ITER) {
     int const g = LAG + pos / ITER, r = pos % ITER;
     return r < UT ? Task{T_U, g - LAG, r} : face_task(g, r - UT);
   }
-  pos -= (IC - LAG) * ITER;
-  if (pos < LAG * UT) return Task{T_U, IC - LAG + pos / UT, pos % UT};
+  pos -= (NX - LAG) * ITER;
+  if (pos < LAG * UT) return Task{T_U, NX - LAG + pos / UT, pos % UT};
   return Task{T_NONE, 0, 0};
 }
 
@@ -128,21 +135,24 @@ __host__ __device__ inline Task decode(int pos) {
 // cell, and for the block's own planes 9 + 9 (y, z faces) + 8 (stage update).
 // A plane with no reads is not loaded; when a plane's count drops to zero its
 // ring slot takes the next loaded plane of that slot.
+template <int NX = IC>
 __host__ __device__ inline void plane_reads(int nlo, int nhi, int (&reads)[NPLANES]) {
   for (int q = 0; q < NPLANES; ++q) reads[q] = 0;
-  for (int a = 0; a <= IC; ++a)
-    for (int m = 0; m < 6; ++m) reads[stencil_src(a - 3 + m, nlo, nhi).index + 3] += XT;
-  for (int g = 0; g < IC; ++g) reads[g + 3] += 2 * YT + UT;
+  for (int a = 0; a <= NX; ++a)
+    for (int m = 0; m < 6; ++m) reads[stencil_src(a - 3 + m, nlo, nhi, NX).index + 3] += XT;
+  for (int g = 0; g < NX; ++g) reads[g + 3] += 2 * YT + UT;
 }
 // First loaded plane of ring slot s (or 99 when none).
+template <int NX = IC>
 __host__ __device__ inline int first_plane_of_slot(int s, int const (&reads)[NPLANES]) {
-  for (int q = s - 3; q <= IC + 2; q += RING)
+  for (int q = s - 3; q <= NX + 2; q += RING)
     if (reads[q + 3] > 0) return q;
   return 99;
 }
 // The loaded plane after q in q's ring slot (or 99 when none).
+template <int NX = IC>
 __host__ __device__ inline int next_plane_of_slot(int q, int const (&reads0)[NPLANES]) {
-  for (int n = q + RING; n <= IC + 2; n += RING)
+  for (int n = q + RING; n <= NX + 2; n += RING)
     if (reads0[n + 3] > 0) return n;
   return 99;
 }
@@ -155,21 +165,30 @@ __host__ __device__ inline int next_plane_of_slot(int q, int const (&reads0)[NPL
 struct Box {
   int k, j, i, blk;
 };
-// Plane q (-3..18) of block `slot`: box 16 (z) x 16 (y) x 1 (x) x 5 fields.
-__host__ __device__ inline Box plane_box(int q, int slot, int const (&nbr)[6]) {
-  if (q < 0) return Box{HS, HS, HS + q + IC, nbr[0]};
-  if (q >= IC) return Box{HS, HS, HS + q - IC, nbr[1]};
-  return Box{HS, HS, HS + q, slot};
+// Plane q (-3 .. NX + 2) of the item at plane x0 of block `slot`: box 16 (z) x 16
+// (y) x 1 (x) x 5 fields.
+__host__ __device__ inline Box plane_box(int q, int slot, int const (&nbr)[6], int x0 = 0) {
+  int const x = x0 + q;
+  if (x < 0) return Box{HS, HS, HS + x + IC, nbr[0]};
+  if (x >= IC) return Box{HS, HS, HS + x - IC, nbr[1]};
+  return Box{HS, HS, HS + x, slot};
 }
 // y halo rows of plane g: rows 13..15 of the low neighbour (side 0), 0..2 of
 // the high one (side 1); box 16 x 3 x 1 x 5.
-__host__ __device__ inline Box yhalo_box(int g, int side, int const (&nbr)[6]) {
-  return Box{HS, side ? HS : HS + IC - 3, HS + g, nbr[2 + side]};
+__host__ __device__ inline Box yhalo_box(int g, int side, int const (&nbr)[6], int x0 = 0) {
+  return Box{HS, side ? HS : HS + IC - 3, HS + x0 + g, nbr[2 + side]};
 }
 // z halo columns of plane g: columns 12..15 of the low neighbour, 0..3 of the
 // high one; box 4 x 16 x 1 x 5.
-__host__ __device__ inline Box zhalo_box(int g, int side, int const (&nbr)[6]) {
-  return Box{side ? HS : HS + IC - 4, HS, HS + g, nbr[4 + side]};
+__host__ __device__ inline Box zhalo_box(int g, int side, int const (&nbr)[6], int x0 = 0) {
+  return Box{side ? HS : HS + IC - 4, HS, HS + x0 + g, nbr[4 + side]};
+}
+// Neighbours of the item at plane x0: a part's inner x neighbour is the block
+// itself.
+template <int NX>
+__host__ __device__ inline void item_neighbours(int x0, int slot, int (&nbr)[6]) {
+  if (x0 > 0) nbr[0] = slot;
+  if (x0 + NX < IC) nbr[1] = slot;
 }
 
 // ---- shared memory of one CTA ------------------------------------------------
@@ -197,6 +216,7 @@ struct Smem {
   int next_task;
   int item, skip, bad, dt_ready;
   int nbr[6];
+  int x0;  // the item's first plane
   double dt;
   double red[32];
 };
@@ -247,6 +267,7 @@ __host__ __device__ inline void gather_interior(double const *p, double (&cons)[
 // canonical order) of face q of x face plane g (dir 0) or of plane g (dir 1,
 // 2), from the ring and the halo buffers; symmetry walls negate the principal
 // momentum of mirrored cells.
+template <int NX = IC>
 __host__ __device__ inline void gather_face(Smem const &S, int dir, int g, int w, int q,
                                             double (&cons)[6][NE]) {
   FaceAt const f = face_at(dir, q);
@@ -269,7 +290,7 @@ __host__ __device__ inline void gather_face(Smem const &S, int dir, int g, int w
   int const hfs = dir == 1 ? YROW : ZCOL;
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
-    Src const s = stencil_src(a - 3 + m, nlo, nhi);
+    Src const s = stencil_src(a - 3 + m, nlo, nhi, dir == 0 ? NX : IC);
     double const *src;
     int fs;
     if (dir == 0) {  // uniform over the warp

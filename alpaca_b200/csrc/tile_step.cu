@@ -10,18 +10,28 @@
 
 namespace alp {
 
-extern template cudaError_t tile_kernel_info<FV_CHAR>(int, int, TileKernelInfo *);
-extern template cudaError_t tile_kernel_info<FV_PRIM>(int, int, TileKernelInfo *);
-extern template cudaError_t tile_kernel_info<FS_ROE>(int, int, TileKernelInfo *);
+extern template cudaError_t tile_kernel_info<FV_CHAR>(int, int, int, TileKernelInfo *);
+extern template cudaError_t tile_kernel_info<FV_PRIM>(int, int, int, TileKernelInfo *);
+extern template cudaError_t tile_kernel_info<FS_ROE>(int, int, int, TileKernelInfo *);
 
-cudaError_t tile_info(int scheme, int variant, int precision, TileKernelInfo *out) {
+cudaError_t tile_info(int scheme, int variant, int planes, int precision, TileKernelInfo *out) {
   if (variant < 0 || variant >= kTileVariants) return cudaErrorInvalidValue;
   switch (scheme) {
-    case FV_CHAR: return tile_kernel_info<FV_CHAR>(variant, precision, out);
-    case FV_PRIM: return tile_kernel_info<FV_PRIM>(variant, precision, out);
-    case FS_ROE: return tile_kernel_info<FS_ROE>(variant, precision, out);
+    case FV_CHAR: return tile_kernel_info<FV_CHAR>(variant, planes, precision, out);
+    case FV_PRIM: return tile_kernel_info<FV_PRIM>(variant, planes, precision, out);
+    case FS_ROE: return tile_kernel_info<FS_ROE>(variant, planes, precision, out);
   }
   return cudaErrorInvalidValue;
+}
+
+// Parts as long as they find idle CTAs: a part computes the x face at its inner
+// end as well and fills its pipeline anew. Step of FV char in ms, whole blocks /
+// halves / quarters: 1 block 0.396 / 0.215 / 0.126, 8: 0.401 / 0.218 / 0.127, 27:
+// 0.427 / 0.241 / 0.131; whole blocks / halves: 60 blocks 0.463 / 0.243, 100: 0.475
+// / 0.363, 125: 0.471 / 0.431, 148: 0.471 / 0.474, 224: 0.730 / 0.745, 512: 1.63 /
+// 1.65.
+int tile_parts(int nwork, int ctas) {
+  return 4 * nwork <= ctas ? 4 : (nwork < ctas ? 2 : 1);
 }
 
 namespace {

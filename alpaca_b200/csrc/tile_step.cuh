@@ -1,8 +1,8 @@
 // Fused 3D stepping kernel: one persistent launch advances every resident case
 // of an engine n SSP-RK3 (or TVD-RK2) steps.
 //
-// Work items are (step, stage, block) in a fixed order; each CTA takes the next
-// item from a device counter. An item
+// Work items are (step, stage, block, part of the block's x-planes) in a fixed
+// order; each CTA takes the next item from a device counter. An item
 //   1. waits (thread 0, bounded) until its block and its six face neighbours
 //      have finished the previous stage (per-block flags, release / acquire);
 //   2. streams the stage input into shared memory with TMA
@@ -100,6 +100,9 @@ __device__ __forceinline__ int ld_acquire(int const *p) {
 __device__ __forceinline__ void st_release(int *p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ void add_release(int *p, int v) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 // Bounded spin of a warp until *p >= v (global, another CTA's release); on
 // running out sets err bit `code` and returns.
 __device__ __forceinline__ void spin_ge(int const *p, int v, int *err, int code) {
@@ -121,7 +124,7 @@ constexpr unsigned kZBytes = NE * ZCOL * sizeof(double);
 // or the x neighbour's plane beyond the face.
 __device__ __forceinline__ void issue_plane(Smem &S, CUtensorMap const *map, int slot, int q) {
   unsigned long long *b = &S.bar_plane[q + 3];
-  Box const x = plane_box(q, slot, S.nbr);
+  Box const x = plane_box(q, slot, S.nbr, S.x0);
   mbar_expect(b, kPlaneBytes);
   tma_load(&S.ring[ring_slot(q)][0][0], map, x.k, x.j, x.i, 0, x.blk, b);
 }
@@ -139,7 +142,7 @@ __device__ __forceinline__ void issue_halos(Smem &S, CUtensorMap const *ymap,
                          (nb >= 0 ? kZBytes : 0) + (nt >= 0 ? kZBytes : 0);
   mbar_expect(b, bytes);
   for (int side = 0; side < 2; ++side) {
-    Box const y = yhalo_box(g, side, S.nbr), z = zhalo_box(g, side, S.nbr);
+    Box const y = yhalo_box(g, side, S.nbr, S.x0), z = zhalo_box(g, side, S.nbr, S.x0);
     if (y.blk >= 0) tma_load(&S.yh[hb][side][0][0], ymap, y.k, y.j, y.i, 0, y.blk, b);
     if (z.blk >= 0) tma_load(&S.zh[hb][side][0][0], zmap, z.k, z.j, z.i, 0, z.blk, b);
   }
@@ -147,13 +150,13 @@ __device__ __forceinline__ void issue_halos(Smem &S, CUtensorMap const *ymap,
 
 __device__ __forceinline__ void issue_u0(Smem &S, CUtensorMap const *map, int slot, int g) {
   mbar_expect(&S.bar_u0[g], kPlaneBytes);
-  tma_load(&S.u0[g % BU][0][0], map, HS, HS, HS + g, 0, slot, &S.bar_u0[g]);
+  tma_load(&S.u0[g % BU][0][0], map, HS, HS, HS + S.x0 + g, 0, slot, &S.bar_u0[g]);
 }
 
 // ---- tasks -----------------------------------------------------------------
 struct ItemCtx {
   CUtensorMap const *pmap, *ymap, *zmap, *u0map;
-  double *out;  // the block in the stage output pool
+  double *out;  // the item's first plane's block origin in the stage output pool
   int slot, stage, step;
   bool first, reduce;
   Eos eos;
@@ -189,7 +192,7 @@ __device__ __forceinline__ int vol(int const &x) { return *reinterpret_cast<int 
 // lanes side by side. Every direction goes through the one face_compute<3, 0>
 // of the rotated stencil (gather_face), so the SM runs one copy of the face
 // arithmetic.
-template <int SCHEME, typename T>
+template <int SCHEME, typename T, int NX>
 __device__ __forceinline__ void task_face(Smem &S, ItemCtx const &C, Task const &t, bool compute) {
   int const lane = threadIdx.x & 31;
   int const dir = t.type;  // T_FX, T_FY, T_FZ are 0, 1, 2
@@ -203,7 +206,7 @@ __device__ __forceinline__ void task_face(Smem &S, ItemCtx const &C, Task const 
         [&] {
           if (lane == 0) return g <= RFX || mbar_try(&S.bar_u[g - RFX - 1]);
           if (lane == 1) return g < RFX || mbar_try(&S.bar_u[g - RFX]);
-          if (lane < 8) return mbar_try(&S.bar_plane[stencil_src(g - 5 + lane, nlo, nhi).index + 3]);
+          if (lane < 8) return mbar_try(&S.bar_plane[stencil_src(g - 5 + lane, nlo, nhi, NX).index + 3]);
           return true;
         },
         C.err, 2);
@@ -223,7 +226,7 @@ __device__ __forceinline__ void task_face(Smem &S, ItemCtx const &C, Task const 
   int const q = t.w * 32 + lane;
   if (compute && face_at(dir, q).valid) {
     double cons[6][NE];
-    gather_face(S, dir, g, t.w, q, cons);
+    gather_face<NX>(S, dir, g, t.w, q, cons);
     double fd[NE];
     bool const valid = face_compute<3, 0, SCHEME, T>(C.eos, C.B, cons, fd);
     FluxAt const o = flux_at(S, dir, g, q);
@@ -237,9 +240,9 @@ __device__ __forceinline__ void task_face(Smem &S, ItemCtx const &C, Task const 
     if (lane == 0) {
       mbar_arrive(&S.bar_x[g]);
     } else if (lane < 7) {
-      int const pq = stencil_src(g - 4 + lane, S.nbr[0], S.nbr[1]).index;
+      int const pq = stencil_src(g - 4 + lane, S.nbr[0], S.nbr[1], NX).index;
       if (atomicSub(&S.reads[pq + 3], 1) == 1) {
-        int const n = next_plane_of_slot(pq, S.reads0);
+        int const n = next_plane_of_slot<NX>(pq, S.reads0);
         if (n != 99) issue_plane(S, C.pmap, C.slot, n);
       }
     }
@@ -248,11 +251,11 @@ __device__ __forceinline__ void task_face(Smem &S, ItemCtx const &C, Task const 
       mbar_arrive(&S.bar_yz[g]);
     } else if (lane == 1) {
       if (atomicSub(&S.reads[g + 3], 1) == 1) {
-        int const n = next_plane_of_slot(g, S.reads0);
+        int const n = next_plane_of_slot<NX>(g, S.reads0);
         if (n != 99) issue_plane(S, C.pmap, C.slot, n);
       }
     } else if (lane == 2) {
-      if (atomicSub(&S.reads_h[g], 1) == 1 && g + BH < IC) issue_halos(S, C.ymap, C.zmap, g + BH);
+      if (atomicSub(&S.reads_h[g], 1) == 1 && g + BH < NX) issue_halos(S, C.ymap, C.zmap, g + BH);
     }
   }
   __syncwarp();
@@ -260,6 +263,7 @@ __device__ __forceinline__ void task_face(Smem &S, ItemCtx const &C, Task const 
 
 // Stage update of 32 cells of plane g: flux divergence and RK stage into the
 // output; the last stage also takes the cells' signal speed.
+template <int NX>
 __device__ __forceinline__ void task_u(Smem &S, ItemCtx const &C, int g, int w, double &smax,
                                        int &bad) {
   int const lane = threadIdx.x & 31;
@@ -310,19 +314,20 @@ __device__ __forceinline__ void task_u(Smem &S, ItemCtx const &C, int g, int w, 
     mbar_arrive(&S.bar_u[g]);
   } else if (lane == 1) {
     if (atomicSub(&S.reads[g + 3], 1) == 1) {
-      int const n = next_plane_of_slot(g, S.reads0);
+      int const n = next_plane_of_slot<NX>(g, S.reads0);
       if (n != 99) issue_plane(S, C.pmap, C.slot, n);
     }
   } else if (lane == 2 && !first) {
-    if (atomicSub(&S.reads_u[g], 1) == 1 && g + BU < IC) issue_u0(S, C.u0map, C.slot, g + BU);
+    if (atomicSub(&S.reads_u[g], 1) == 1 && g + BU < NX) issue_u0(S, C.u0map, C.slot, g + BU);
   }
   __syncwarp();
 }
 
 }  // namespace tile
 
-// The persistent kernel: NW warps, one CTA per SM (shared memory).
-template <int SCHEME, typename T, int NW>
+// The persistent kernel: NW warps, one CTA per SM (shared memory), NX x-planes of
+// a block per item (16, or 8 or 4: two or four items per block and stage).
+template <int SCHEME, typename T, int NW, int NX>
 __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__ const TileArgs A) {
   using namespace tile;
   // no static shared memory: the dynamic block starts the CTA's shared window,
@@ -331,7 +336,9 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Smem &S = *reinterpret_cast<Smem *>(smem_raw);
   int const tid = threadIdx.x, lane = tid & 31;
-  int const per_step = A.nstages * A.nwork;
+  constexpr int PARTS = IC / NX;  // items per block and stage
+  int const per_stage = A.nwork * PARTS;
+  int const per_step = A.nstages * per_stage;
   int const total = per_step * A.nsteps;
   int *err = A.ctrl + 1;
   if (smem_addr(smem_raw) & 127) {
@@ -350,11 +357,16 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
     int const item = S.item;
     if (item >= total) break;
     int const step = item / per_step;
-    int const s = (item / A.nwork) % A.nstages;
-    int const slot = A.order[s * A.nwork + item % A.nwork];
+    int const s = (item / per_stage) % A.nstages;
+    int const in_stage = item % per_stage;
+    int const slot = A.order[s * A.nwork + in_stage / PARTS];
+    int const x0 = (in_stage % PARTS) * NX;
     int const stage = A.stage0 + s;
     bool const last = s == A.nstages - 1;
-    int const need = A.nstages * step + s;
+    // finished items of a block before this stage; a block's parts are never more
+    // than one stage apart (a part at stage n starts it only once the sum is
+    // PARTS n, which one lagging part prevents), so the sum tells each of them
+    int const need = PARTS * (A.nstages * step + s);
     // stage input / output pools: RK3 A -> B, (B, A) -> C, (C, A) -> A;
     // RK2 A -> B, (B, A) -> A; a trial's last stage writes B (RK3) or C (RK2)
     int const pin = s;
@@ -378,6 +390,8 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
     if (tid == 0) {
       int const *nb = A.nbr26 + (size_t)slot * 26;
       for (int d = 0; d < 6; ++d) S.nbr[d] = nb[face_slot(d)];
+      item_neighbours<NX>(x0, slot, S.nbr);
+      S.x0 = x0;
       // dt of this step: final for later stages; for a first stage only once
       // the previous step's last blocks of the case committed
       int const ready = s > 0 || ld_acquire(A.dtflag + cid) >= step + 1;
@@ -388,9 +402,9 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
       S.bad = 0;
       S.next_task = 0;
       int reads[NPLANES];
-      plane_reads(S.nbr[0], S.nbr[1], reads);
+      plane_reads<NX>(S.nbr[0], S.nbr[1], reads);
       for (int q = 0; q < NPLANES; ++q) S.reads[q] = S.reads0[q] = reads[q];
-      for (int g = 0; g < IC; ++g) {
+      for (int g = 0; g < NX; ++g) {
         S.reads_h[g] = 2 * YT;
         S.reads_u[g] = UT;
       }
@@ -401,11 +415,11 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
         if (bars_live) mbar_inval(&S.bar_plane[q]);
         mbar_init(&S.bar_plane[q]);
       }
-      for (int g = 0; g <= IC; ++g) {
+      for (int g = 0; g <= NX; ++g) {
         if (bars_live) mbar_inval(&S.bar_x[g]);
         mbar_init(&S.bar_x[g], XT);
       }
-      for (int g = 0; g < IC; ++g) {
+      for (int g = 0; g < NX; ++g) {
         if (bars_live) {
           mbar_inval(&S.bar_halo[g]);
           mbar_inval(&S.bar_u0[g]);
@@ -424,7 +438,7 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
         asm volatile("fence.proxy.async;" ::: "memory");
         CUtensorMap const *pmap = &A.plane[pin];
         for (int r = 0; r < RING; ++r) {
-          int const q = first_plane_of_slot(r, reads);
+          int const q = first_plane_of_slot<NX>(r, reads);
           if (q != 99) issue_plane(S, pmap, slot, q);
         }
         for (int g = 0; g < BH; ++g) issue_halos(S, &A.yhalo[pin], &A.zhalo[pin], g);
@@ -441,7 +455,7 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
       C.ymap = &A.yhalo[pin];
       C.zmap = &A.zhalo[pin];
       C.u0map = &A.plane[0];
-      C.out = A.pool[pout] + (size_t)slot * Geo<3>::BLOCK_DOUBLES;
+      C.out = A.pool[pout] + (size_t)slot * Geo<3>::BLOCK_DOUBLES + x0 * Geo<3>::cell(1, 0, 0);
       C.slot = slot;
       C.stage = stage;
       C.step = step;
@@ -462,14 +476,14 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
       if (lane == 0) pos = atomicAdd(&S.next_task, 1);
       pos = __shfl_sync(kFull, pos, 0);
 #pragma unroll 1
-      while (pos < STREAM) {
+      while (pos < stream_length<NX>()) {
         int claim = 0;
         if (lane == 0) claim = atomicAdd(&S.next_task, 1);
-        Task const t = decode(pos);
+        Task const t = decode<NX>(pos);
         // a first stage whose dt turned out 0 keeps the bookkeeping, skips the work
         bool const compute = !*reinterpret_cast<int volatile *>(&S.skip);
-        if (t.type == T_U) task_u(S, C, t.g, t.w, smax, bad);
-        else if (t.type != T_NONE) task_face<SCHEME, T>(S, C, t, compute);
+        if (t.type == T_U) task_u<NX>(S, C, t.g, t.w, smax, bad);
+        else if (t.type != T_NONE) task_face<SCHEME, T, NX>(S, C, t, compute);
         pos = __shfl_sync(kFull, claim, 0);
       }
       __syncthreads();
@@ -491,11 +505,11 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
     __syncthreads();
     if (tid == 0) {
       __threadfence();
-      st_release(A.done + slot, need + 1);
+      add_release(A.done + slot, 1);
       if (last) {
         // the case's last block of this step commits it and computes the next dt
         int const old = atomicAdd(A.cnt + cid, 1);
-        if (old == (step + 1) * A.case_nb[cid] - 1) {
+        if (old == (step + 1) * A.case_nb[cid] * PARTS - 1) {
           __threadfence();
           if (!A.trial) {
             CaseState volatile *vs = A.cases + cid;
@@ -526,9 +540,9 @@ __global__ void __launch_bounds__(NW * 32, 1) tile_step_kernel(__grid_constant__
 }
 
 namespace tile {
-template <int SCHEME, typename T, int NW>
+template <int SCHEME, typename T, int NW, int NX>
 cudaError_t info_one(TileKernelInfo *out) {
-  void const *fn = reinterpret_cast<void const *>(&tile_step_kernel<SCHEME, T, NW>);
+  void const *fn = reinterpret_cast<void const *>(&tile_step_kernel<SCHEME, T, NW, NX>);
   size_t const smem = sizeof(Smem);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -539,10 +553,14 @@ cudaError_t info_one(TileKernelInfo *out) {
   return cudaSuccess;
 }
 template <int SCHEME, typename T>
-cudaError_t info_t(int variant, TileKernelInfo *out) {
-  switch (variant) {
-    case 0: return info_one<SCHEME, T, 16>(out);
-    case 1: return info_one<SCHEME, T, 12>(out);
+cudaError_t info_t(int variant, int planes, TileKernelInfo *out) {
+  switch (variant * 100 + planes) {
+    case 16: return info_one<SCHEME, T, 16, 16>(out);
+    case 8: return info_one<SCHEME, T, 16, 8>(out);
+    case 4: return info_one<SCHEME, T, 16, 4>(out);
+    case 116: return info_one<SCHEME, T, 12, 16>(out);
+    case 108: return info_one<SCHEME, T, 12, 8>(out);
+    case 104: return info_one<SCHEME, T, 12, 4>(out);
   }
   return cudaErrorInvalidValue;
 }
@@ -550,9 +568,9 @@ cudaError_t info_t(int variant, TileKernelInfo *out) {
 
 // Sets the kernel's shared-memory limit and reports its launch shape.
 template <int SCHEME>
-cudaError_t tile_kernel_info(int variant, int precision, TileKernelInfo *out) {
-  return precision == FP32_FLUX ? tile::info_t<SCHEME, float>(variant, out)
-                                : tile::info_t<SCHEME, double>(variant, out);
+cudaError_t tile_kernel_info(int variant, int planes, int precision, TileKernelInfo *out) {
+  return precision == FP32_FLUX ? tile::info_t<SCHEME, float>(variant, planes, out)
+                                : tile::info_t<SCHEME, double>(variant, planes, out);
 }
 
 }  // namespace alp

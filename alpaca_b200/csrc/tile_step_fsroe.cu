@@ -3,5 +3,6 @@
 #include "tile_step.cuh"
 
 namespace alp {
-template cudaError_t tile_kernel_info<FS_ROE>(int variant, int precision, TileKernelInfo *out);
+template cudaError_t tile_kernel_info<FS_ROE>(int variant, int planes, int precision,
+                                                     TileKernelInfo *out);
 }  // namespace alp
