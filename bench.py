@@ -37,9 +37,9 @@ B_ALG_3D = 320.0  # algorithmic HBM bytes per 3D cell-update (64 * N_eq, FP64 st
 FLOPS_PER_CELL_UPDATE_3D = {"fvchar": 15767, "fvprim": 10192, "fsroe": 22478}
 FLOPS_PER_CELL_UPDATE_2D = {"fvchar": 8004, "fvprim": 5448, "fsroe": 10605}
 # DRAM bytes per SSP-RK3 step of the 128^3 workload (sum of dram__bytes_read.sum
-# and dram__bytes_write.sum over the step's kernels, one ncu capture; summary in
+# and dram__bytes_write.sum over the step's kernels under ncu; summary in
 # profiles/step_fvchar_128cubed.md)
-TRAFFIC_PER_STEP = {("fvchar", "fp64"): 4.359e9}
+TRAFFIC_PER_STEP = {("fvchar", "fp64"): 3.279e9}
 # DRAM bytes per cell-update of the multi-level step (fvchar, FP64): one ncu
 # capture of a macro step of the same hierarchy at n0 = 2 (31 / 264 leaves, 176
 # ghosts, 4.58 M cell-updates, 9.38 GB), scaled by cell-updates (summary in

@@ -391,8 +391,10 @@ int alp_engine_set_graph(alp_engine *e, int enabled);
 #define ALP_STEP_CANDIDATES 6
 
 /* Times the stepping candidates on the engine's resident cases and keeps the
- * fastest: 0 = face fluxes (128-thread blocks, all directions in one launch)
- * + divergence/stage update, 1 = the same with 64-thread blocks, 2 = pencil
+ * fastest: 0 = face fluxes (128-thread blocks; with many blocks the last
+ * direction fused with the divergence/stage update, else all directions in one
+ * launch and the update in another; small 1D and 2D work lists take whole steps
+ * in one thread-block cluster), 1 = the same with 64-thread blocks, 2 = pencil
  * sweeps (one thread per line of cells, 17 faces with a sliding stencil
  * window, flux differences summed in the kernels and the RK stage applied by
  * the last direction; not available in the strict build; default schemes
@@ -401,7 +403,8 @@ int alp_engine_set_graph(alp_engine *e, int enabled);
  * arithmetic), 4 = fused tile stages with 16 warps per CTA, 5 = the same with
  * 12 warps. The fused tile stages (3D engines with WENO5 + HLLC/Einfeldt or
  * Roe splitting, RK3 or RK2) advance all steps of one alp_engine_step call in
- * one persistent launch: per (step, stage, block) work item, the block's cell
+ * one persistent launch: per (step, stage, block) work item (halves or quarters
+ * of a block while CTAs would idle otherwise), its cell
  * planes and the neighbours' cells beyond its faces are staged into shared
  * memory by TMA, every face flux is computed once into shared memory and the
  * divergence and RK stage are applied there, so no face flux reaches HBM. Its
@@ -420,8 +423,9 @@ int alp_engine_set_path(alp_engine *e, int candidate);
 /* The engine's current stepping candidate (-1 for a null engine). */
 int alp_engine_path(alp_engine *e);
 
-/* Number of kernel launches one engine step issues (the fused tile stages:
- * per alp_engine_step call, whatever its step count). */
+/* Number of kernel launches one engine step issues (the fused tile stages and
+ * small 1D and 2D work lists: per alp_engine_step call, see
+ * alp_engine_launches). */
 int alp_engine_launches_per_step(alp_engine *e);
 
 /* Number of kernel launches alp_engine_step(e, n) issues. */
