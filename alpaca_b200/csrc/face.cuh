@@ -251,9 +251,9 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
         return valid;
       }
       double const one_l = inv(cm[MASS]), one_r = inv(cp[MASS]);
-      double const pm = eos_pressure<DIM>(eos, cm[MASS], cm[MOMX], DIM > 1 ? cm[MOMX + (DIM > 1)] : 0.0,
+      double const pm = eos_pressure<DIM, false>(eos, cm[MASS], cm[MOMX], DIM > 1 ? cm[MOMX + (DIM > 1)] : 0.0,
                                           DIM > 2 ? cm[MOMX + 2 * (DIM > 2)] : 0.0, cm[ENERGY], one_l);
-      double const pp = eos_pressure<DIM>(eos, cp[MASS], cp[MOMX], DIM > 1 ? cp[MOMX + (DIM > 1)] : 0.0,
+      double const pp = eos_pressure<DIM, false>(eos, cp[MASS], cp[MOMX], DIM > 1 ? cp[MOMX + (DIM > 1)] : 0.0,
                                           DIM > 2 ? cp[MOMX + 2 * (DIM > 2)] : 0.0, cp[ENERGY], one_r);
       if (!(pm > -B) || !(pp > -B)) valid = false;
       hllc_mixed<DIM, DIR>(eos, cm, cp, pm, pp, cm[mP] * one_l, cp[mP] * one_r, one_l, one_r, fd);
@@ -287,11 +287,11 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
       // prime states of the reconstructed states (prime_state_handler.h:277-371),
       // pressure recovered in double
       T const one_l = inv(cm[MASS]), one_r = inv(cp[MASS]);
-      double const pm = eos_pressure<DIM>(eos, double(cm[MASS]), double(cm[MOMX]),
+      double const pm = eos_pressure<DIM, false>(eos, double(cm[MASS]), double(cm[MOMX]),
                                           DIM > 1 ? double(cm[MOMX + (DIM > 1)]) : 0.0,
                                           DIM > 2 ? double(cm[MOMX + 2 * (DIM > 2)]) : 0.0,
                                           double(cm[ENERGY]), double(one_l));
-      double const pp = eos_pressure<DIM>(eos, double(cp[MASS]), double(cp[MOMX]),
+      double const pp = eos_pressure<DIM, false>(eos, double(cp[MASS]), double(cp[MOMX]),
                                           DIM > 1 ? double(cp[MOMX + (DIM > 1)]) : 0.0,
                                           DIM > 2 ? double(cp[MOMX + 2 * (DIM > 2)]) : 0.0,
                                           double(cp[ENERGY]), double(one_r));
@@ -354,7 +354,7 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
 #pragma unroll
       for (int m = 0; m < W; ++m) {
         double const one_rho = inv(cons[m][MASS]);
-        double const p = eos_pressure<DIM>(
+        double const p = eos_pressure<DIM, false>(
             eos, cons[m][MASS], cons[m][MOMX], DIM > 1 ? cons[m][MOMX + (DIM > 1)] : 0.0,
             DIM > 2 ? cons[m][MOMX + 2 * (DIM > 2)] : 0.0, cons[m][ENERGY], one_rho);
         double const vel = cons[m][mP] * one_rho;
@@ -432,13 +432,13 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
         // velocities, then the pressure with the kinetic energy u . m / 2
         prim[m][RHO] = cons[m][MASS];
         double const one = inv(cons[m][MASS]);
-        double um = 0.0;
+        double v[DIM], mom[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
-          prim[m][VELX + d] = cons[m][MOMX + d] * one;
-          um = d == 0 ? prim[m][VELX] * cons[m][MOMX]
-                      : fma(prim[m][VELX + d], cons[m][MOMX + d], um);
+          mom[d] = cons[m][MOMX + d];
+          prim[m][VELX + d] = v[d] = mom[d] * one;
         }
+        double um = axis_dot<DIM, DIR>(v, mom);
         if (eos.safe && !(cons[m][MASS] > DBL_EPSILON)) um *= cons[m][MASS] * (1.0 / DBL_EPSILON);
         double p = fma(eos.gamma - 1.0, fma(-0.5, um, cons[m][ENERGY]), -(eos.gamma * eos.B));
         if (eos.safe) p = dmax(p, -eos.B + DBL_EPSILON);

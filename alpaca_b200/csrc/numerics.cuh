@@ -120,11 +120,29 @@ template <int DIM, typename T> __device__ __forceinline__ T dacms(T a, T b, T c)
   else return cms3(a, b, c);
 }
 
-// Sum of three squares: DimensionAwareConsistencyManagedSum in the strict build;
-// the fast build adds them in order.
-template <int DIM, typename T> __device__ __forceinline__ T sum_sq(T a, T b, T c) {
-  if constexpr (!ALP_FAST || DIM < 3) return dacms<DIM>(a, b, c);
-  else return (a + b) + c;
+// Sum of three squares: DimensionAwareConsistencyManagedSum in the strict build
+// and in 1D / 2D. The fast build's 3D sum is independent of the order of its
+// terms as well: it sorts them (the bit patterns of non-negative floating-point
+// values order like the values) and adds the two smaller first, two additions and
+// integer compares against seven additions and four floating-point compares, so
+// that prime states, energies, signal speeds (dt) and the primitive form do not
+// change when the axes are exchanged. ORDERED = false adds them as they come, for
+// the characteristic forms, whose projections follow an order anyway.
+template <int DIM, bool ORDERED = true, typename T>
+__device__ __forceinline__ T sum_sq(T a, T b, T c) {
+  if constexpr (!ALP_FAST || DIM < 3) {
+    return dacms<DIM>(a, b, c);
+  } else if constexpr (!ORDERED) {
+    return (a + b) + c;
+  } else {
+    static_assert(sizeof(T) == 8, "the FP32-flux form sums floats unordered");
+    long long const ia = __double_as_longlong(a), ib = __double_as_longlong(b);
+    long long const ic = __double_as_longlong(c);
+    long long const lo = min(ia, ib), hi = max(ia, ib);
+    long long const x0 = min(lo, ic), t = max(lo, ic);
+    long long const x1 = min(t, hi), x2 = max(t, hi);
+    return (__longlong_as_double(x0) + __longlong_as_double(x1)) + __longlong_as_double(x2);
+  }
 }
 
 // ---- stiffened gas (generic_stiffened_gas.h:40-102, stiffened_gas.cpp:62-149,
@@ -135,19 +153,20 @@ struct Eos {
   int safe;
 };
 
-// one_mass = inv(mass) (unused by the strict build, which divides)
-template <int DIM>
+// one_mass = inv(mass) (unused by the strict build, which divides); ORDERED as in
+// sum_sq
+template <int DIM, bool ORDERED = true>
 __device__ __forceinline__ double eos_pressure(Eos const &e, double mass, double mx, double my,
                                                double mz, double energy, double one_mass) {
   if (e.safe) {
     double const m = dmax(mass, DBL_EPSILON);
     double const p =
         -e.gamma * e.B +
-        (e.gamma - 1.0) * (energy - quot(0.5 * sum_sq<DIM>(mx * mx, my * my, mz * mz), m,
+        (e.gamma - 1.0) * (energy - quot(0.5 * sum_sq<DIM, ORDERED>(mx * mx, my * my, mz * mz), m,
                                          mass > DBL_EPSILON ? one_mass : inv(m)));
     return dmax(p, -e.B + DBL_EPSILON);
   }
-  double const q = 0.5 * sum_sq<DIM>(mx * mx, my * my, mz * mz);
+  double const q = 0.5 * sum_sq<DIM, ORDERED>(mx * mx, my * my, mz * mz);
   return -e.gamma * e.B + (e.gamma - 1.0) * (energy - quot(q, mass, one_mass));
 }
 template <int DIM>
@@ -408,7 +427,7 @@ __device__ __forceinline__ CellPrims<DIM, DIR> cell_prims(Eos const &e, double c
   r.up = c[MOMX + DIR] * r.one_rho;
   r.u1 = DIM > 1 ? c[MOMX + (DIM > 1 ? Minor<DIR>::m1 : 0)] * r.one_rho : 0.0;
   r.u2 = DIM > 2 ? c[MOMX + (DIM > 2 ? Minor<DIR>::m2 : 0)] * r.one_rho : 0.0;
-  r.p = eos_pressure<DIM>(e, c[MASS], mx, my, mz, c[ENERGY], r.one_rho);
+  r.p = eos_pressure<DIM, false>(e, c[MASS], mx, my, mz, c[ENERGY], r.one_rho);
   // Enthalpy (stiffened_gas.cpp:88-96 / stiffened_gas_safe.cpp:77-84)
   r.H = e.safe ? quot(c[ENERGY] + r.p, dmax(c[MASS], DBL_EPSILON))
                : quot(c[ENERGY] + r.p, c[MASS], r.one_rho);
@@ -451,9 +470,9 @@ __device__ __forceinline__ Roe<T> roe_average(Eos const &e, CellPrims<DIM, DIR> 
   T const psi = ((psi_t * sr_t) + (psi_n * sr_n)) * rho_div;
   r.H = (T(t.H) * sr_t + T(n.H) * sr_n) * rho_div;
   r.gru = T(e.gamma - 1.0);
-  r.q2 = sum_sq<DIM>(r.up * r.up, r.u1 * r.u1, r.u2 * r.u2);
+  r.q2 = sum_sq<DIM, false>(r.up * r.up, r.u1 * r.u1, r.u2 * r.u2);
   T const dup = T(t.up) - T(n.up), du1 = T(t.u1) - T(n.u1), du2 = T(t.u2) - T(n.u2);
-  T const tmp = sum_sq<DIM>(dup * dup, du1 * du1, du2 * du2);
+  T const tmp = sum_sq<DIM, false>(dup * dup, du1 * du1, du2 * du2);
   // 0.5 rho_roe rho_div^2 = 0.5 w_t w_n
   T const jump = WEIGHTS ? T(0.5) * (sr_t * sr_n) * tmp
                          : T(0.5) * r.rho * (rho_div * rho_div) * tmp;
@@ -542,10 +561,11 @@ __device__ __forceinline__ void to_physical(Roe<T> const &r, T const (&ch)[DIM +
     if constexpr (DIM == 2) s = ch[1] * (-r.u1 * r.rho);
     if constexpr (DIM > 2) {
       // The two minor-wave terms are rounded as products before they are
-      // added, so that the sum does not depend on which minor momentum is
-      // numbered first: with the minor momenta exchanged (and their waves'
-      // signs, as the characteristic variables then are) the bits are the
-      // same. The strict build rounds every product anyway.
+      // added, so that this sum does not depend on which minor momentum is
+      // numbered first (rotate.cuh numbers those of y faces the other way
+      // round). The strict build rounds every product anyway; the fast build's
+      // projection adds its terms in an order, so its characteristic fluxes
+      // still change at rounding level when the minor momenta are exchanged.
       T const t1 = rmul(ch[1], -r.u1 * r.rho);
       T const t2 = rmul(ch[2], r.rho * r.u2);
       s = t1 + t2;
@@ -579,7 +599,7 @@ __device__ __forceinline__ void to_physical_packed(Roe<float> const &r, float2 c
   if constexpr (DIM == 2) s = fma2(ch[1], dup2(-r.u1 * r.rho), s);
   if constexpr (DIM > 2) {
     // the two minor-wave products rounded before they are added, as in
-    // to_physical (the same bits with the minor momenta exchanged)
+    // to_physical
     s = add2(add2(mul2(ch[1], dup2(-r.u1 * r.rho)), mul2(ch[2], dup2(r.rho * r.u2))), s);
   }
   out[ENERGY] = s;
@@ -806,6 +826,19 @@ __device__ __forceinline__ void hllc_flux(HllcUpwind const &h, double const (&cl
   }
 }
 
+// Sum of a[d] b[d] over the axes, the principal one fused onto the sum of the two
+// minor products, each rounded on its own: the same bits with the minor axes
+// exchanged (the fast build's primitive form; one operation more than a chain).
+template <int DIM, int DIR>
+__device__ __forceinline__ double axis_dot(double const (&a)[DIM], double const (&b)[DIM]) {
+  if constexpr (DIM == 1) return a[0] * b[0];
+  else if constexpr (DIM == 2) return fma(a[DIR], b[DIR], rmul(a[1 - DIR], b[1 - DIR]));
+  else
+    return fma(a[DIR], b[DIR],
+               rmul(a[Minor<DIR>::m1], b[Minor<DIR>::m1]) +
+                   rmul(a[Minor<DIR>::m2], b[Minor<DIR>::m2]));
+}
+
 // Its flux from prime states (Density, Pressure, VelocityX..): the upwind side's
 // conserved quantities alone.
 template <int DIM, int DIR>
@@ -814,13 +847,13 @@ __device__ __forceinline__ void hllc_flux_primes(Eos const &e, HllcUpwind const 
                                                  double const (&pp)[DIM + 2],
                                                  double (&flux)[DIM + 2]) {
   flux[MASS] = h.rho * h.k;
-  double q = 0.0;
+  double v[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
-    double const v = h.right ? pp[VELX + d] : pm[VELX + d];
-    q = d == 0 ? v * v : fma(v, v, q);
-    flux[MOMX + d] = d == DIR ? fma(h.rho, h.g, h.p) : v * flux[MASS];
+    v[d] = h.right ? pp[VELX + d] : pm[VELX + d];
+    flux[MOMX + d] = d == DIR ? fma(h.rho, h.g, h.p) : v[d] * flux[MASS];
   }
+  double const q = axis_dot<DIM, DIR>(v, v);
   double const E = fma(0.5 * h.rho, q, (h.p + e.gamma * e.B) * inv(e.gamma - 1.0));
   flux[ENERGY] = fma(E, h.k, h.pe);
 }
