@@ -97,8 +97,10 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
           for (int n = 0; n < NE; ++n) G[n][m] = ch[n];
         }
         double il[NE], ir[NE];
+        double const minor = dmax(r.rho2, kMinorRho2);
 #pragma unroll
-        for (int n = 0; n < NE; ++n) pol.increments(G[n], char_scale<DIM>(r, n), il[n], ir[n]);
+        for (int n = 0; n < NE; ++n)
+          pol.increments(G[n], char_scale<DIM>(minor, n), il[n], ir[n], minor_wave<DIM>(n));
         double cm[NE], cp[NE];
         char_restore<DIM, DIR>(r, cons[C], il, 1.0, cm);
         char_restore<DIM, DIR>(r, cons[C + 1], ir, -1.0, cp);
@@ -147,13 +149,29 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
 #pragma unroll
           for (int l = 0; l < NE; ++l) fa[l] = fb[l];
         }
+        MinorUnits const mu = minor_units(r.rho2);
+        if (DIM > 1 && __builtin_expect(mu.tiny, 0)) {
+#pragma unroll
+          for (int n = 1; n < DIM; ++n) {
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+              if (m < 4) A[n][m] *= mu.unit;
+              if (m > 0) N[n][m] *= mu.unit;
+            }
+            w[n] *= mu.unit;
+          }
+        }
 #pragma unroll
         for (int n = 0; n < NE; ++n) {
           double l, q;
           A[n][4] = 0.0;
           N[n][0] = 0.0;
-          pol.increments_two(A[n], N[n], char_scale<DIM>(r, n), l, q);
+          pol.increments_two(A[n], N[n], char_scale<DIM>(mu.scale, n), l, q, minor_wave<DIM>(n));
           w[n] = 0.5 * ((l - q) - w[n]);
+        }
+        if (DIM > 1 && __builtin_expect(mu.tiny, 0)) {
+#pragma unroll
+          for (int n = 1; n < DIM; ++n) w[n] *= mu.back;
         }
         char_restore<DIM, DIR>(r, fi, w, 1.0, fd);
       }
@@ -512,7 +530,7 @@ __device__ __forceinline__ bool face_compute(Eos const &eos, double B,
           double G[5], l, r;
 #pragma unroll
           for (int m = 0; m < 5; ++m) G[m] = prim[m + 1][n] - prim[m][n];
-          pol.increments(G, 1.0, l, r);
+          pol.increments(G, 1.0, l, r, false);
           pm[n] = prim[C][n] + l;
           pp[n] = prim[C + 1][n] - r;
         } else {

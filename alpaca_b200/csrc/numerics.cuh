@@ -273,11 +273,18 @@ __device__ __forceinline__ Weno5Frac weno5_frac(double g2, double g3, double d1,
   return {fma(y, fma(z, r2, t2 * r3), p * r1), fma(y, z + t2, p)};
 }
 
-// num_l / (6 den_l) and num_r / (6 den_r) with one reciprocal: the denominators
-// lie between ~1e-23 (eps^4) and ~1e2 |g|^8, so their product stays in range
-// for differences up to ~1e17.
+// num_l / (6 den_l) and num_r / (6 den_r). One reciprocal serves both while the
+// product of the denominators, each between ~1e-23 (eps^4) and ~1e2 |g|^8, stays
+// in range: for differences up to ~1e17 and the reference's eps. `apart` takes a
+// reciprocal per side, for differences up to ~1e38 and eps down to ~1e-77 (one
+// operation more).
 __device__ __forceinline__ void weno5_finish(Weno5Frac const &l, Weno5Frac const &r,
-                                             double &left, double &right) {
+                                             double &left, double &right, bool apart) {
+  if (apart) {
+    left = l.num * inv(6.0 * l.den);
+    right = r.num * inv(6.0 * r.den);
+    return;
+  }
   double const rr = inv((6.0 * l.den) * r.den);
   left = l.num * (r.den * rr);
   right = r.num * (l.den * rr);
@@ -289,21 +296,22 @@ __device__ __forceinline__ void weno5_finish(Weno5Frac const &l, Weno5Frac const
 // factor by which the caller scaled the differences (WENO5 of scaled data with
 // eps scaled alike is the scaled WENO5).
 __device__ __forceinline__ void weno5_increments(double const (&G)[5], double eps, double &left,
-                                                 double &right) {
+                                                 double &right, bool apart) {
   double const D1 = G[1] - G[0], D2 = G[2] - G[1], D3 = G[3] - G[2], D4 = G[4] - G[3];
   double const q2 = weno5_q(D2, eps), q3 = weno5_q(D3, eps);
   weno5_finish(weno5_frac(G[1], G[2], D1, D3, weno5_q(D1, eps), q2, q3),
-               weno5_frac(G[3], G[2], -D4, -D2, weno5_q(D4, eps), q3, q2), left, right);
+               weno5_frac(G[3], G[2], -D4, -D2, weno5_q(D4, eps), q3, q2), left, right, apart);
 }
 // The same for two arrays (flux splitting): UpwindLeft from the differences
 // A[0..3], UpwindRight from B[1..4].
 __device__ __forceinline__ void weno5_increments_two(double const (&A)[5], double const (&B)[5],
-                                                     double eps, double &left, double &right) {
+                                                     double eps, double &left, double &right,
+                                                     bool apart) {
   double const A1 = A[1] - A[0], A2 = A[2] - A[1], A3 = A[3] - A[2];
   double const B2 = B[2] - B[1], B3 = B[3] - B[2], B4 = B[4] - B[3];
   weno5_finish(weno5_frac(A[1], A[2], A1, A3, weno5_q(A1, eps), weno5_q(A2, eps), weno5_q(A3, eps)),
                weno5_frac(B[3], B[2], -B4, -B2, weno5_q(B4, eps), weno5_q(B3, eps), weno5_q(B2, eps)),
-               left, right);
+               left, right, apart);
 }
 
 // ---- packed FP32 pairs (Blackwell f32x2: one instruction for two lanes) ----
@@ -356,7 +364,7 @@ __device__ __forceinline__ void weno5_pair(T const (&a)[6], T &left, T &right) {
   } else {
     double const G[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], a[5] - a[4]};
     double l, r;
-    weno5_increments(G, 1.0e-6, l, r);
+    weno5_increments(G, 1.0e-6, l, r, false);
     left = a[2] + l;
     right = a[3] - r;
   }
@@ -373,7 +381,7 @@ __device__ __forceinline__ void weno5_two(T const (&a)[6], T const (&b)[6], T &l
     double const A[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], 0.0};
     double const B[5] = {0.0, b[2] - b[1], b[3] - b[2], b[4] - b[3], b[5] - b[4]};
     double l, r;
-    weno5_increments_two(A, B, 1.0e-6, l, r);
+    weno5_increments_two(A, B, 1.0e-6, l, r, false);
     left = a[2] + l;
     right = b[3] - r;
   }
@@ -725,10 +733,44 @@ __device__ __forceinline__ void char_project(CharFrame<DIM> const &r, double con
   ch[DIM + 1] = fma(r.one_c, Dp, s);
 }
 
-// Square of the factor on the characteristic values of wave n in these scales.
+// Whether wave n is one of the minor waves.
+template <int DIM> __host__ __device__ constexpr bool minor_wave(int n) {
+  return n > 0 && n < DIM;
+}
+
+// The minor waves' values carry a factor rho_roe: momentum-sized, they span more
+// than the other waves' values, so their reconstruction takes a reciprocal per side
+// (weno5_finish). Where the product rho2 of the densities is below kMinorRho2, the
+// fourth power of its eps would leave the double range all the same.
+constexpr double kMinorRho2 = 1.0e-60;
+
+// Square of the factor on the characteristic values of wave n in these scales,
+// minor_scale that of the minor waves.
 template <int DIM>
-__device__ __forceinline__ double char_scale(CharFrame<DIM> const &r, int n) {
-  return n == 0 || n == DIM + 1 ? 4.0 : (n == DIM ? 1.0 : r.rho2);
+__device__ __forceinline__ double char_scale(double minor_scale, int n) {
+  return n == 0 || n == DIM + 1 ? 4.0 : (n == DIM ? 1.0 : minor_scale);
+}
+
+// Flux splitting takes any positive density: below the line the minor waves'
+// values are multiplied by `unit`, a power of two near 1 / rho_roe, for their
+// reconstruction. (The finite-volume forms refuse reconstructed densities below
+// 2.2e-16 and keep kMinorRho2 as the least scale: on the faces they accept that
+// changes the weights of minor values below 1e-33 only, nothing beside the momenta
+// of such densities. The branch cost FV char 3 % through its registers, flux
+// splitting 1 %.)
+struct MinorUnits {
+  double scale, unit, back;
+  bool tiny;
+};
+__device__ __forceinline__ MinorUnits minor_units(double rho2) {
+  MinorUnits u{rho2, 1.0, 1.0, !(rho2 > kMinorRho2)};
+  if (__builtin_expect(u.tiny, 0)) {
+    int const h = (1023 - ((__double2hiint(rho2) >> 20) & 0x7ff)) / 2;
+    u.unit = __hiloint2double((1023 + h) << 20, 0);
+    u.back = __hiloint2double((1023 - h) << 20, 0);
+    u.scale = (rho2 * u.unit) * u.unit;
+  }
+  return u;
 }
 
 // base + sgn (the conserved difference whose scaled characteristic values are ch).

@@ -176,9 +176,10 @@ __device__ __forceinline__ void stencil_increments(double const (&A)[5], double 
     double const eps = S::EPS * scale;
     Weno5Frac const l = S::make(A[0], A[1], A[2], A[3], eps);
     Weno5Frac const r = S::make(B[4], B[3], B[2], B[1], eps);
-    double const rr = inv((S::FACTOR * l.den) * r.den);
-    left = l.num * (r.den * rr);
-    right = r.num * (l.den * rr);
+    // a reciprocal per side: the denominators' product leaves the double range
+    // for differences above ~1e19 (WENO5) that each side by itself can hold
+    left = l.num * inv(S::FACTOR * l.den);
+    right = r.num * inv(S::FACTOR * r.den);
   }
 }
 
@@ -385,13 +386,15 @@ __device__ __forceinline__ void riemann_ext(int solver, int speeds, Eos const &e
 // stencil (CharFrame), reconstructed by increments / increments_two.
 struct DefaultPolicy {
   static constexpr bool FAST_FRAME = true;
+  // apart: as in weno5_finish
   __device__ __forceinline__ void increments(double const (&G)[5], double scale, double &l,
-                                             double &r) const {
-    weno5_increments(G, 1.0e-6 * scale, l, r);
+                                             double &r, bool apart) const {
+    weno5_increments(G, 1.0e-6 * scale, l, r, apart);
   }
   __device__ __forceinline__ void increments_two(double const (&A)[5], double const (&B)[5],
-                                                 double scale, double &l, double &r) const {
-    weno5_increments_two(A, B, 1.0e-6 * scale, l, r);
+                                                 double scale, double &l, double &r,
+                                                 bool apart) const {
+    weno5_increments_two(A, B, 1.0e-6 * scale, l, r, apart);
   }
   __host__ __device__ static constexpr bool default_riemann() { return true; }
   template <int DIM>
@@ -440,11 +443,11 @@ template <int ST> struct ExtPolicy {
   SchemeOptions o;
   double glf[3] = {0.0, 0.0, 0.0};  // GlobalLaxFriedrichs wave speeds of the block's case
   __device__ __forceinline__ void increments(double const (&G)[5], double scale, double &l,
-                                             double &r) const {
+                                             double &r, bool) const {
     stencil_increments<ST>(G, G, scale, l, r);
   }
   __device__ __forceinline__ void increments_two(double const (&A)[5], double const (&B)[5],
-                                                 double scale, double &l, double &r) const {
+                                                 double scale, double &l, double &r, bool) const {
     stencil_increments<ST>(A, B, scale, l, r);
   }
   __device__ __forceinline__ bool default_riemann() const {
