@@ -639,7 +639,7 @@ int alp_engine_step(alp_engine *e, int n) {
   if (n <= 0 || e->nwork == 0) return ALP_OK;
   // profiler ranges (no cost unless a tool is attached): one per call, one per capture
   nvtx3::scoped_range range{"alp_engine_step"};
-  if (e->path == 3) return e->run_tiles(n);
+  if (e->path == 3) return e->step_tiles(n, false);
   if (e->small_steps()) return e->record_step(false, n);
   if (!e->use_graph) {
     for (int i = 0; i < n; ++i)
@@ -835,7 +835,7 @@ int alp_engine_autotune(alp_engine *e, int trial_steps, int *chosen, float *ms_p
     if (!cand_refusal(e, i) && e->nwork > 0) {
       select_cand(e, i);
       auto trial = [&](int n) {
-        if (e->path == 3) return e->record_tiles(n, true);
+        if (e->path == 3) return e->step_tiles(n, true);
         for (int k = 0; k < n; ++k)
           if (int rc = e->record_step(true)) return rc;
         return (int)ALP_OK;
@@ -906,7 +906,10 @@ int alp_engine_launches_per_step(alp_engine *e) {
 
 int alp_engine_launches(alp_engine *e, int n) {
   if (!e || n <= 0 || e->nwork == 0) return 0;
-  if (e->path == 3) return 3;
+  if (e->path == 3) {
+    int const most = e->tile_max_steps();
+    return 3 * (n / most + (n % most != 0));
+  }
   return e->small_steps() ? small_launches(n) : n * alp_engine_launches_per_step(e);
 }
 

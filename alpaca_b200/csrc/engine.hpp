@@ -178,9 +178,25 @@ struct alp_engine {
     return ALP_OK;
   }
 
+  // Steps one persistent launch of path 3 may run on the current work list.
+  int tile_max_steps() const {
+    return alp::tile_max_steps(nwork, rk2 ? 2 : 3, tgrid[tile_variant]);
+  }
+
+  // Path 3: n steps, in as many launches as their item count needs.
+  int step_tiles(int n, bool trial) {
+    int const most = tile_max_steps();
+    for (; n > 0; n -= std::min(n, most)) {
+      int const m = std::min(n, most);
+      if (int rc = trial ? record_tiles(m, true) : run_tiles(m)) return rc;
+    }
+    return ALP_OK;
+  }
+
   // Path 3: the dt of the first step (signal speed, dt_finalize, which marks
-  // it ready), then one persistent launch for n steps (tile_step.cuh); the
-  // flags and counters of the launch start at zero, the error word is kept.
+  // it ready), then one persistent launch for n <= tile_max_steps() steps
+  // (tile_step.cuh); the flags and counters of the launch start at zero, the
+  // error word is kept.
   int record_tiles(int n, bool trial) {
     if (nwork == 0 || n <= 0) return ALP_OK;
     int *dtflag = tsync + 2 + slots_max;

@@ -49,6 +49,8 @@ cudaError_t tile_kernel_info(int variant, int planes, int precision, TileKernelI
 cudaError_t tile_info(int scheme, int variant, int planes, int precision, TileKernelInfo *out);
 // Items per block (1, 2 or 4) with which nwork blocks step fastest on `ctas` CTAs.
 int tile_parts(int nwork, int ctas);
+// Steps one launch may run on nwork blocks (longer calls launch several times).
+int tile_max_steps(int nwork, int nstages, int ctas);
 // TMA descriptors of the three block pools (reference layout, `capacity`
 // blocks each) into a; false with a reason when the driver cannot encode them.
 bool tile_encode(TileArgs &a, double *const pools[3], int capacity, std::string &why);

@@ -191,6 +191,14 @@ __host__ __device__ inline void item_neighbours(int x0, int slot, int (&nbr)[6])
   if (x0 + NX < IC) nbr[1] = slot;
 }
 
+// Steps one launch may run: work items are numbered in 32 bits, over all its steps
+// and past the last item by one per CTA.
+__host__ __device__ inline int max_steps_per_launch(int nwork, int parts, int nstages, int ctas) {
+  long long const per_step = (long long)nwork * parts * nstages;
+  long long const n = per_step > 0 ? (0x7fffffffLL - ctas) / per_step : 0x7fffffffLL;
+  return n < 1 ? 1 : (int)n;
+}
+
 // ---- shared memory of one CTA ------------------------------------------------
 struct Smem {
   double ring[RING][NE][PLANE];

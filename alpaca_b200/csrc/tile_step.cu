@@ -7,6 +7,7 @@
 
 #include "kernels.cuh"
 #include "tile_api.cuh"
+#include "tile_plan.cuh"
 
 namespace alp {
 
@@ -32,6 +33,10 @@ cudaError_t tile_info(int scheme, int variant, int planes, int precision, TileKe
 // 1.65.
 int tile_parts(int nwork, int ctas) {
   return 4 * nwork <= ctas ? 4 : (nwork < ctas ? 2 : 1);
+}
+
+int tile_max_steps(int nwork, int nstages, int ctas) {
+  return tile::max_steps_per_launch(nwork, tile_parts(nwork, ctas), nstages, ctas);
 }
 
 namespace {

@@ -403,7 +403,8 @@ int alp_engine_set_graph(alp_engine *e, int enabled);
  * arithmetic), 4 = fused tile stages with 16 warps per CTA, 5 = the same with
  * 12 warps. The fused tile stages (3D engines with WENO5 + HLLC/Einfeldt or
  * Roe splitting, RK3 or RK2) advance all steps of one alp_engine_step call in
- * one persistent launch: per (step, stage, block) work item (halves or quarters
+ * one persistent launch (several beyond 2^31 work items): per (step, stage,
+ * block) work item (halves or quarters
  * of a block while CTAs would idle otherwise), its cell
  * planes and the neighbours' cells beyond its faces are staged into shared
  * memory by TMA, every face flux is computed once into shared memory and the
