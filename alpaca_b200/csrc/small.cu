@@ -143,7 +143,7 @@ bool small_pays(int dim, int nwork) {
   return dim < 3 && stage_faces(dim, nwork) <= kSmallCtas * kSmallThreads;
 }
 
-int small_launches(int n) { return (n + kSmallSteps - 1) / kSmallSteps; }
+int small_launches(int n) { return n / kSmallSteps + (n % kSmallSteps != 0); }
 
 cudaError_t launch_small_steps(Launch const &L, double *const in[3], double *const out[3],
                                double *F, long long stride, long long dstride, int const *nbr26,
@@ -200,8 +200,8 @@ cudaError_t launch_small_steps(Launch const &L, double *const in[3], double *con
       cfg.gridDim = dim3(8);
     }
   }
-  for (int done = 0; done < n; done += kSmallSteps) {
-    a.nsteps = n - done < kSmallSteps ? n - done : kSmallSteps;
+  for (; n > 0; n -= a.nsteps) {
+    a.nsteps = n < kSmallSteps ? n : kSmallSteps;
     void *args[] = {&a};
     if (cudaError_t e = cudaLaunchKernelExC(&cfg, k, args)) return e;
   }

@@ -22,3 +22,14 @@ def test_tile_launches(cuda, n, parts):
     assert [e.launches(k) for k in (1, most, most + 1)] == [3, 3, 6]
     assert e.launches(MOST) == 3 * -(-MOST // most)
     e.close()
+
+
+@pytest.mark.parametrize("dim,n", [(1, (8, 1, 1)), (2, (2, 2, 1))])
+def test_small_launches(cuda, dim, n):
+    """Small 1D and 2D lists: a launch per 256 steps."""
+    c = box(dim, n, True, 32)
+    e = api.Engine(dim, "fvchar", capacity_blocks=c.grid.nb, max_cases=1)
+    e.add_case(c)
+    assert [e.launches(k) for k in (1, 256, 257, 512)] == [1, 1, 2, 2]
+    assert e.launches(MOST) == 2 ** 23
+    e.close()
