@@ -836,6 +836,7 @@ int alp_engine_autotune(alp_engine *e, int trial_steps, int *chosen, float *ms_p
       select_cand(e, i);
       auto trial = [&](int n) {
         if (e->path == 3) return e->step_tiles(n, true);
+        if (e->small_steps()) return e->record_step(true, n);  // as alp_engine_step runs them
         for (int k = 0; k < n; ++k)
           if (int rc = e->record_step(true)) return rc;
         return (int)ALP_OK;
