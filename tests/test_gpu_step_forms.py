@@ -48,8 +48,7 @@ def same(a, b):
         assert s == sv and t == tv and np.array_equal(u, v)
 
 
-# 3D from 128 blocks, 2D from 1200 blocks; uneven counts, so that the last warps
-# of the launch have no lines
+# 3D from 128 blocks, 2D from 1200 blocks: 8 lines to a warp at these counts
 @pytest.mark.parametrize("scheme,precision", [("fvchar", N.FP64), ("fvprim", N.FP64),
                                               ("fsroe", N.FP64), ("fvchar", N.FP32_FLUX),
                                               ("fsroe", N.FP32_FLUX), ("fvchar_weno3_hll", N.FP64),
@@ -63,6 +62,33 @@ def test_sweep_matches_plain_form(cuda, scheme, precision, dim, n, edge):
     steps = [3, 2][:len(cs)]
     a, _ = run(dim, cs, scheme, precision, 0, steps)
     b, _ = run(dim, cs, scheme, precision, PLAIN, steps)
+    same(a, b)
+
+
+@pytest.fixture(scope="module")
+def large():
+    """Boxes of the larger sweeps, built once."""
+    built = {}
+
+    def get(dim, n, edge):
+        if (dim, n) not in built:
+            built[dim, n] = box(dim, n, edge, 8)
+        return built[dim, n]
+    return get
+
+
+# 16 lines to a warp from 444 3D blocks and from 7104 2D blocks, 32 from 888 3D
+# blocks, where every lane computes a line's last face; an odd number of 2D blocks
+# leaves the last warp of the launch without lines
+@pytest.mark.parametrize("scheme,precision", [("fvchar", N.FP64), ("fvprim", N.FP64),
+                                              ("fsroe", N.FP64), ("fvchar", N.FP32_FLUX),
+                                              ("fvchar_weno3_hll", N.FP64)])
+@pytest.mark.parametrize("dim,n,edge", [(3, (10, 9, 5), True), (3, (10, 9, 10), False),
+                                        (2, (35, 203, 1), True)])
+def test_longer_sweeps_match_plain_form(cuda, large, scheme, precision, dim, n, edge):
+    cs = [large(dim, n, edge)]
+    a, _ = run(dim, cs, scheme, precision, 0, [2])
+    b, _ = run(dim, cs, scheme, precision, PLAIN, [2])
     same(a, b)
 
 
