@@ -31,7 +31,8 @@ namespace alp {
 // Reciprocal by one third-order Householder iteration on f(y) = 1/y - b
 // (Householder 1970: y <- y (1 + e + e^2), e = 1 - b y), seeded with the PTX
 // approximate reciprocal: the seed's ~2^-20 relative error becomes its cube,
-// 2^-60, in three operations (two Newton steps: four).
+// 2^-60, in three operations (two Newton steps: four), so that the rounding of
+// the last operation is all that is left. For 2^-1022 <= |b| <= 2^1022.
 __device__ __forceinline__ double rcp_nr(double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
@@ -41,8 +42,9 @@ __device__ __forceinline__ double rcp_nr(double b) {
 
 // 1/sqrt(x) by one third-order Householder iteration on f(y) = 1/y^2 - x
 // (y <- y (1 + e/2 + 3 e^2/8), e = 1 - x y^2), seeded with the PTX approximate
-// reciprocal square root (fast build only); the remaining error is 5/16 e^3,
-// below 2^-58.
+// reciprocal square root (fast build only). The iteration leaves 5/16 e^3, below
+// 2^-58; the rounding of x y in e, half of which reaches y, and that of the last
+// operation are larger. For normal x.
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

@@ -1,6 +1,9 @@
-// Measurement helpers for bench.py (not part of the C ABI of the engine):
-// the FP64 FMA-pipe peak of the device, measured with independent DFMA chains.
+// Measurement helpers for bench.py and the tests (not part of the C ABI of the
+// engine): the FP64 FMA-pipe peak of the device, measured with independent DFMA
+// chains, and the refined reciprocals of the fast build.
 #include <cuda_runtime.h>
+
+#include "numerics.cuh"
 
 namespace {
 
@@ -20,7 +23,21 @@ __global__ void __launch_bounds__(256) dfma_chains(double a, double b, int iters
   if (s == 12345.678) out[0] = s;  // keeps the chains live
 }
 
+__global__ void reciprocals(double const *x, double *rcp, double *rsqrt, int n) {
+  int const i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  rcp[i] = alp::rcp_nr(x[i]);
+  rsqrt[i] = alp::rsqrt_nr(fabs(x[i]));
+}
+
 }  // namespace
+
+// rcp[i] = rcp_nr(x[i]), rsqrt[i] = rsqrt_nr(|x[i]|); device arrays of n.
+extern "C" int alp_probe_reciprocals(double const *x, double *rcp, double *rsqrt, int n) {
+  if (n <= 0) return 0;
+  reciprocals<<<(n + 255) / 256, 256>>>(x, rcp, rsqrt, n);
+  return cudaDeviceSynchronize() == cudaSuccess ? 0 : 2;
+}
 
 extern "C" int alp_probe_fp64_peak(int iters, int ctas_per_sm, double *tflops) {
   int dev = 0, sms = 0;
