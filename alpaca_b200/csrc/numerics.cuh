@@ -9,10 +9,11 @@
 // Two builds share this file. The strict build (ALP_STRICT, compiled with
 // -fmad=false) evaluates every expression exactly as the reference writes it,
 // IEEE division included, and reproduces the reference bit for bit. The fast
-// build replaces divisions by Newton-refined reciprocals (reused where the same
-// divisor recurs), evaluates the WENO5 weights of a face's two reconstructions
-// with shared second differences and one reciprocal, and takes float square
-// roots from the hardware approximation; all change results only at the
+// build replaces divisions and square roots by refined reciprocals (one
+// third-order step each, reused where the same divisor recurs), projects and
+// reconstructs the differences of the stencil, evaluates the WENO5 weights of a
+// face's two reconstructions with shared second differences, and takes float
+// square roots from the hardware approximation; all change results only at the
 // rounding level.
 #pragma once
 
@@ -199,6 +200,7 @@ template <typename T> __device__ __forceinline__ T eos_speed_of_sound(Eos const 
 }
 
 // ---- WENO5-JS (stencils/spatial_reconstruction_stencils/weno5.h:88-158) --
+// As the reference writes it: the strict build's form.
 // a[0..5] are cells i-2..i+3 around face i+1/2; UpwindLeft uses {offset 0,
 // sign +1}, UpwindRight {1, -1} (stencils/apply_wrapper.h:47-57).
 template <typename T>
@@ -220,23 +222,14 @@ __device__ __forceinline__ T weno5_core(T v1, T v2, T v3, T v4, T v5) {
   T const t1 = (s1 + eps) * (s1 + eps);
   T const t2 = (s2 + eps) * (s2 + eps);
   T const t3 = (s3 + eps) * (s3 + eps);
-  if constexpr (ALP_FAST && sizeof(T) == 8) {
-    // alpha_k = d_k / t_k scaled by t1 t2 t3: one reciprocal instead of four
-    // divisions (t_k >= 1e-12 and the products stay far inside the double range)
-    T const b1 = T(0.1) * (t2 * t3);
-    T const b2 = T(0.6) * (t1 * t3);
-    T const b3 = T(0.3) * (t1 * t2);
-    return (b1 * q1 + b2 * q2 + b3 * q3) * inv(b1 + b2 + b3);
-  } else {
-    T const a1 = quot(T(0.1), t1);
-    T const a2 = quot(T(0.6), t2);
-    T const a3 = quot(T(0.3), t3);
-    T const one_a_sum = quot(T(1.0), a1 + a2 + a3);
-    T const w1 = a1 * one_a_sum;
-    T const w2 = a2 * one_a_sum;
-    T const w3 = a3 * one_a_sum;
-    return w1 * q1 + w2 * q2 + w3 * q3;
-  }
+  T const a1 = quot(T(0.1), t1);
+  T const a2 = quot(T(0.6), t2);
+  T const a3 = quot(T(0.3), t3);
+  T const one_a_sum = quot(T(1.0), a1 + a2 + a3);
+  T const w1 = a1 * one_a_sum;
+  T const w2 = a2 * one_a_sum;
+  T const w3 = a3 * one_a_sum;
+  return w1 * q1 + w2 * q2 + w3 * q3;
 }
 template <typename T> __device__ __forceinline__ T weno5_left(T const (&a)[6]) {
   return weno5_core(a[0], a[1], a[2], a[3], a[4]);
@@ -354,39 +347,6 @@ __device__ __forceinline__ float2 weno5_packed(float2 g1, float2 g2, float2 g3, 
   float2 const num = fma2(y, fma2(z, r2, mul2(u2, r3)), mul2(p, r1));
   float2 const q = mul2(dup2(6.0f), fma2(y, add2(z, u2), p));
   return mul2(num, make_float2(inv(q.x), inv(q.y)));
-}
-
-// UpwindLeft and UpwindRight of one face from the same six cells a[0..5]
-// (i-2..i+3).
-template <typename T>
-__device__ __forceinline__ void weno5_pair(T const (&a)[6], T &left, T &right) {
-  if constexpr (!ALP_FAST) {
-    left = weno5_left(a);
-    right = weno5_right(a);
-  } else {
-    double const G[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], a[5] - a[4]};
-    double l, r;
-    weno5_increments(G, 1.0e-6, l, r, false);
-    left = a[2] + l;
-    right = a[3] - r;
-  }
-}
-
-// UpwindLeft of a and UpwindRight of b (flux splitting: the positive and
-// negative split fluxes).
-template <typename T>
-__device__ __forceinline__ void weno5_two(T const (&a)[6], T const (&b)[6], T &left, T &right) {
-  if constexpr (!ALP_FAST) {
-    left = weno5_left(a);
-    right = weno5_right(b);
-  } else {
-    double const A[5] = {a[1] - a[0], a[2] - a[1], a[3] - a[2], a[4] - a[3], 0.0};
-    double const B[5] = {0.0, b[2] - b[1], b[3] - b[2], b[4] - b[3], b[5] - b[4]};
-    double l, r;
-    weno5_increments_two(A, B, 1.0e-6, l, r, false);
-    left = a[2] + l;
-    right = b[3] - r;
-  }
 }
 
 // ---- Roe eigensystem (solvers/eigendecomposition.h:181-467) --------------
@@ -905,18 +865,12 @@ __device__ __forceinline__ void hllc_flux_primes(Eos const &e, HllcUpwind const 
 // CalculateSignalSpeed, Einfeldt (hll_signal_speed_calculator.h:77-101) and
 // HllcRiemannSolver::SolveRiemannProblemImplementation (hllc_riemann_solver.h:52-198)
 // one_rl, one_rr: 1/density of the two states as returned by inv()
+// As the reference writes it: the strict build's form.
 template <int DIM, int DIR, typename T>
-__device__ __forceinline__ void hllc(Eos const &e, T const (&cl)[DIM + 2], T const (&cr)[DIM + 2],
-                                     T pres_l, T pres_r, T vel_l, T vel_r, T one_rl, T one_rr,
-                                     T (&flux)[DIM + 2]) {
-  constexpr int NE = DIM + 2;
+__device__ __forceinline__ void hllc_ordered(Eos const &e, T const (&cl)[DIM + 2],
+                                             T const (&cr)[DIM + 2], T pres_l, T pres_r, T vel_l,
+                                             T vel_r, T one_rl, T one_rr, T (&flux)[DIM + 2]) {
   constexpr int mP = MOMX + DIR;
-  if constexpr (ALP_FAST && sizeof(T) == 8) {
-    hllc_flux<DIM, DIR>(hllc_upwind(e, cl[MASS], cr[MASS], pres_l, pres_r, vel_l, vel_r, one_rl,
-                                    one_rr),
-                        cl, cr, flux);
-    return;
-  }
   T const c_l = eos_speed_of_sound<T>(e, cl[MASS], pres_l, one_rl);
   T const c_r = eos_speed_of_sound<T>(e, cr[MASS], pres_r, one_rr);
   T const srl = tsqrt(cl[MASS]);
@@ -970,7 +924,18 @@ __device__ __forceinline__ void hllc(Eos const &e, T const (&cl)[DIM + 2], T con
     T const fsr = vel_r * cr[mm] + (sr * (chi_r * cr[mm] - cr[mm]));
     flux[mm] = wl * fsl + wr * fsr;
   }
-  (void)NE;
+}
+
+template <int DIM, int DIR, typename T>
+__device__ __forceinline__ void hllc(Eos const &e, T const (&cl)[DIM + 2], T const (&cr)[DIM + 2],
+                                     T pres_l, T pres_r, T vel_l, T vel_r, T one_rl, T one_rr,
+                                     T (&flux)[DIM + 2]) {
+  if constexpr (ALP_FAST)
+    hllc_flux<DIM, DIR>(hllc_upwind(e, cl[MASS], cr[MASS], pres_l, pres_r, vel_l, vel_r, one_rl,
+                                    one_rr),
+                        cl, cr, flux);
+  else
+    hllc_ordered<DIM, DIR, T>(e, cl, cr, pres_l, pres_r, vel_l, vel_r, one_rl, one_rr, flux);
 }
 
 // hllc_upwind of the FP32-flux form: wave speeds, the contact speed and the

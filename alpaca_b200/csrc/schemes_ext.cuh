@@ -183,9 +183,6 @@ __device__ __forceinline__ void stencil_increments(double const (&A)[5], double 
   }
 }
 
-// Reconstruction of the 6-cell array a (cells i-2..i+3 around face i+1/2) with
-// UpwindLeft (right = false) or UpwindRight evaluation properties
-// (stencils/apply_wrapper.h:47-57); narrower stencils use the middle cells.
 // WENO7-JS (weno7.h:21-212; coefficients of Balsara & Shu 2000): v1..v7 the
 // cells i-3..i+3 seen from the upwind side, eps 1e-10, the reference's
 // association order.
@@ -225,9 +222,11 @@ __device__ __forceinline__ double weno7_core(double v1, double v2, double v3, do
          w4 * (3.0 / 12.0 * v4 + 13.0 / 12.0 * v5 + -5.0 / 12.0 * v6 + 1.0 / 12.0 * v7);
 }
 
-// a: the N cells of the stencil line with the face's left cell i at N/2 - 1
-// (N = 6: i-2..i+3, N = 8: i-3..i+4); the five- and three-point stencils read
-// the middle cells.
+// Reconstruction of the N-cell array a around face i+1/2 (N = 6: i-2..i+3, N = 8:
+// i-3..i+4) with UpwindLeft (right = false) or UpwindRight evaluation properties
+// (stencils/apply_wrapper.h:47-57); the five- and three-point stencils read the
+// middle cells. The fast build reaches WENO7 alone here (stencil_increments has the
+// others).
 template <int N>
 __device__ __forceinline__ double reconstruct(int stencil, double const (&a)[N], bool right) {
   constexpr int o = N / 2 - 3;  // a[o + k]: cell i - 2 + k
@@ -405,19 +404,16 @@ struct DefaultPolicy {
     al[1] = fabs(r.up);
     al[2] = fabs(r.up + r.c);
   }
-  template <typename T> __device__ __forceinline__ T left(T const (&a)[6]) const {
-    return weno5_left(a);
-  }
-  template <typename T> __device__ __forceinline__ T right(T const (&a)[6]) const {
-    return weno5_right(a);
-  }
+  // both sides of one array, and of two (the split fluxes): the strict build
   template <typename T>
   __device__ __forceinline__ void pair(T const (&a)[6], T &l, T &r) const {
-    weno5_pair(a, l, r);
+    l = weno5_left(a);
+    r = weno5_right(a);
   }
   template <typename T>
   __device__ __forceinline__ void two(T const (&a)[6], T const (&b)[6], T &l, T &r) const {
-    weno5_two(a, b, l, r);
+    l = weno5_left(a);
+    r = weno5_right(b);
   }
   template <int DIM, int DIR, typename T>
   __device__ __forceinline__ void riemann(Eos const &e, T const (&cl)[DIM + 2],
