@@ -17,7 +17,7 @@ def emu(tmp_path_factory):
     for n in (8, 4):
         out[n] = str(tmp_path_factory.mktemp("tile") / f"tile_plan_part_emu_{n}")
         subprocess.run(["g++", "-O1", "-std=c++17", "-Wno-unknown-pragmas", f"-DNX_PLANES={n}",
-                        "-o", out[n], os.path.join(HERE, "tile_plan_part_emu.cpp")], check=True)
+                        "-o", out[n], os.path.join(HERE, "tile_plan_emu.cpp")], check=True)
     return out
 
 

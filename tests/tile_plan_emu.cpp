@@ -1,16 +1,17 @@
 // CPU replay of the fused tile kernel's plan (alpaca_b200/csrc/tile_plan.cuh)
-// for one work item: the TMA boxes are emulated as copies out of a reference-
-// layout pool, the warp-task stream runs in order with the kernel's
-// bookkeeping (reads counted down, buffers handed to the next plane by their
-// last reader), and every stencil the kernel would read from shared memory is
+// for one work item of NX_PLANES x-planes (16 a whole block, 8 or 4 a part): the
+// TMA boxes are emulated as copies out of a reference-layout pool, the warp-task
+// stream runs in order with the kernel's bookkeeping (reads counted down, buffers
+// handed to the next plane by their last reader), and every stencil the kernel would read from shared memory is
 // compared with the stencil indexed directly in the pool (neighbour interiors,
 // zero gradient or symmetry walls). Buffer contents are tagged so that a stage
 // update reading a flux plane, a ring plane or a U0 plane that was overwritten
 // too early is caught, as is a task whose wait would not be satisfied in
 // stream order (a wait cycle).
 //
-// Usage: tile_plan_emu W E S N B T   (neighbour kinds: 0 periodic neighbour,
-//        1 zero gradient, 2 symmetry); prints "ok <faces> <cells>" or fails.
+// Usage: tile_plan_emu W E S N B T [X0]   (neighbour kinds: 0 periodic neighbour,
+//        1 zero gradient, 2 symmetry; X0: the item's first plane, 0 if absent);
+//        prints "ok <faces> <cells>" or fails.
 #define __host__
 #define __device__
 #include <cmath>
@@ -26,6 +27,10 @@ using namespace alp::tile;
 
 namespace {
 
+#ifndef NX_PLANES
+#define NX_PLANES 16
+#endif
+constexpr int NX = NX_PLANES;  // x-planes of the item
 constexpr int NB = 27;  // a 3 x 3 x 3 block grid; the item is block 13 (the centre)
 constexpr int CELLS = TC * TC * TC;
 std::vector<double> pool;
@@ -54,7 +59,8 @@ void copy_box(double *dst, Box const &x, int ek, int ej) {
 }  // namespace
 
 int main(int argc, char **argv) {
-  if (argc != 7) return 2;
+  if (argc != 7 && argc != 8) return 2;
+  int const x0 = argc == 8 ? std::atoi(argv[7]) : 0;
   int kind[6];
   for (int d = 0; d < 6; ++d) kind[d] = std::atoi(argv[1 + d]);
   // pool: interiors with distinct values, halos NaN (never read)
@@ -68,11 +74,16 @@ int main(int argc, char **argv) {
   int const self = 13;  // (1, 1, 1)
   int nbr[6];
   int const nslot[6] = {13 - 9, 13 + 9, 13 - 3, 13 + 3, 13 - 1, 13 + 1};
-  for (int d = 0; d < 6; ++d) nbr[d] = kind[d] == 0 ? nslot[d] : -kind[d];
+  int real[6];
+  for (int d = 0; d < 6; ++d) real[d] = nbr[d] = kind[d] == 0 ? nslot[d] : -kind[d];
+  item_neighbours<NX>(x0, self, nbr);
 
-  // the expected value of cell c along direction dir (other two interior)
+  // the expected value of cell c along direction dir (other two interior);
+  // along x and across it, planes count from x0
   auto expect = [&](int dir, int c, int p1, int p2, int f) {
-    int const lo = nbr[2 * dir], hi = nbr[2 * dir + 1];
+    if (dir == 0) c += x0;
+    else p1 += x0;
+    int const lo = real[2 * dir], hi = real[2 * dir + 1];
     int blk = self, idx = c;
     bool neg = false;
     if (c < 0) {
@@ -98,6 +109,7 @@ int main(int argc, char **argv) {
   int cnt_x[IC + 1] = {}, cnt_yz[IC] = {}, cnt_u[IC] = {};
   std::memset(&S, 0, sizeof(S));
   for (int d = 0; d < 6; ++d) S.nbr[d] = nbr[d];
+  S.x0 = x0;
   // buffer tags: which plane / face each buffer holds (-100: none)
   int ring_tag[RING], fx_tag[RFX], fyz_tag[BYZ], h_tag[BH], u_tag[BU];
   for (int &t : ring_tag) t = -100;
@@ -108,9 +120,9 @@ int main(int argc, char **argv) {
   bool plane_loaded[NPLANES] = {}, halo_loaded[IC] = {}, u0_loaded[IC] = {};
 
   int reads[NPLANES];
-  plane_reads(nbr[0], nbr[1], reads);
+  plane_reads<NX>(nbr[0], nbr[1], reads);
   for (int q = 0; q < NPLANES; ++q) S.reads[q] = S.reads0[q] = reads[q];
-  for (int g = 0; g < IC; ++g) {
+  for (int g = 0; g < NX; ++g) {
     S.reads_h[g] = 2 * YT;
     S.reads_u[g] = UT;
   }
@@ -120,7 +132,7 @@ int main(int argc, char **argv) {
     int const s = ring_slot(q);
     check(ring_tag[s] == -100 || S.reads[ring_tag[s] + 3] == 0, "ring slot reused early", q,
           ring_tag[s], 0);
-    copy_box(&S.ring[s][0][0], plane_box(q, self, nbr), IC, IC);
+    copy_box(&S.ring[s][0][0], plane_box(q, self, nbr, x0), IC, IC);
     ring_tag[s] = q;
     check(!plane_loaded[q + 3], "plane loaded twice", q, 0, 0);
     plane_loaded[q + 3] = true;
@@ -129,7 +141,7 @@ int main(int argc, char **argv) {
     int const hb = g % BH;
     check(h_tag[hb] == -100 || S.reads_h[h_tag[hb]] == 0, "halo buffer reused early", g, 0, 0);
     for (int side = 0; side < 2; ++side) {
-      Box const y = yhalo_box(g, side, nbr), z = zhalo_box(g, side, nbr);
+      Box const y = yhalo_box(g, side, nbr, x0), z = zhalo_box(g, side, nbr, x0);
       if (y.blk >= 0) copy_box(&S.yh[hb][side][0][0], y, IC, 3);
       if (z.blk >= 0) copy_box(&S.zh[hb][side][0][0], z, 4, IC);
     }
@@ -139,20 +151,20 @@ int main(int argc, char **argv) {
   auto issue_u0 = [&](int g) {
     int const ub = g % BU;
     check(u_tag[ub] == -100 || S.reads_u[u_tag[ub]] == 0, "U0 buffer reused early", g, 0, 0);
-    copy_box(&S.u0[ub][0][0], plane_box(g, self, nbr), IC, IC);
+    copy_box(&S.u0[ub][0][0], plane_box(g, self, nbr, x0), IC, IC);
     u_tag[ub] = g;
     u0_loaded[g] = true;
   };
   auto release_plane = [&](int q) {
     actual_reads[q + 3]++;
     if (--S.reads[q + 3] == 0) {
-      int const n = next_plane_of_slot(q, S.reads0);
+      int const n = next_plane_of_slot<NX>(q, S.reads0);
       if (n != 99) issue_plane(n);
     }
   };
 
   for (int r = 0; r < RING; ++r) {
-    int const q = first_plane_of_slot(r, reads);
+    int const q = first_plane_of_slot<NX>(r, reads);
     if (q != 99) issue_plane(q);
   }
   for (int g = 0; g < BH; ++g) issue_halos(g);
@@ -161,15 +173,15 @@ int main(int argc, char **argv) {
   long faces = 0, cells = 0;
   int covered_x[IC + 1][PLANE] = {}, covered_y[IC][FACE_ROW * IC] = {},
       covered_z[IC][FACE_ROW * IC] = {}, covered_u[IC][PLANE] = {};
-  for (int pos = 0; pos < STREAM; ++pos) {
-    Task const t = decode(pos);
+  for (int pos = 0; pos < stream_length<NX>(); ++pos) {
+    Task const t = decode<NX>(pos);
     if (t.type == T_FX) {
       int const a = t.g;
       // waits: flux slot free, source planes loaded
       if (a > RFX) check(cnt_u[a - RFX - 1] >= UT, "fx wait (a-5) unsatisfied", a, pos, 0);
       if (a >= RFX) check(cnt_u[a - RFX] >= UT, "fx wait (a-4) unsatisfied", a, pos, 0);
       for (int m = 0; m < 6; ++m) {
-        int const q = stencil_src(a - 3 + m, nbr[0], nbr[1]).index;
+        int const q = stencil_src(a - 3 + m, nbr[0], nbr[1], NX).index;
         check(plane_loaded[q + 3], "fx source plane not loaded", a, q, pos);
         check(ring_tag[ring_slot(q)] == q, "fx source slot holds another plane", a, q,
               ring_tag[ring_slot(q)]);
@@ -177,7 +189,7 @@ int main(int argc, char **argv) {
       for (int l = 0; l < 32; ++l) {
         int const jk = t.w * 32 + l;
         double cons[6][NE];
-        gather_face(S, 0, a, t.w, jk, cons);
+        gather_face<NX>(S, 0, a, t.w, jk, cons);
         for (int m = 0; m < 6; ++m)
           for (int c = 0; c < NE; ++c)
             check(cons[m][c] == expect(0, a - 3 + m, jk / IC, jk % IC, canon_field(0, c)),
@@ -189,7 +201,7 @@ int main(int argc, char **argv) {
       }
       fx_tag[a % RFX] = a;
       cnt_x[a]++;
-      for (int m = 0; m < 6; ++m) release_plane(stencil_src(a - 3 + m, nbr[0], nbr[1]).index);
+      for (int m = 0; m < 6; ++m) release_plane(stencil_src(a - 3 + m, nbr[0], nbr[1], NX).index);
     } else if (t.type == T_FY || t.type == T_FZ) {
       int const g = t.g, dir = t.type == T_FY ? 1 : 2;
       if (g >= BYZ) check(cnt_u[g - BYZ] >= UT, "yz buffer wait unsatisfied", g, pos, 0);
@@ -201,7 +213,7 @@ int main(int argc, char **argv) {
         if (!fa.valid) continue;
         int const a = fa.a, tt = fa.t;
         double cons[6][NE];
-        gather_face(S, dir, g, t.w, q, cons);
+        gather_face<NX>(S, dir, g, t.w, q, cons);
         for (int m = 0; m < 6; ++m)
           for (int c = 0; c < NE; ++c) {
             // transverse indices: y faces (x = g, z = tt); z faces (x = g, y = tt);
@@ -220,7 +232,7 @@ int main(int argc, char **argv) {
       fyz_tag[g % BYZ] = g;
       cnt_yz[g]++;
       release_plane(g);
-      if (--S.reads_h[g] == 0 && g + BH < IC) issue_halos(g + BH);
+      if (--S.reads_h[g] == 0 && g + BH < NX) issue_halos(g + BH);
     } else if (t.type == T_U) {
       int const g = t.g;
       check(cnt_x[g] >= XT && cnt_x[g + 1] >= XT && cnt_yz[g] >= 2 * YT,
@@ -233,9 +245,9 @@ int main(int argc, char **argv) {
       for (int l = 0; l < 32; ++l) {
         int const jk = t.w * 32 + l;
         for (int f = 0; f < NE; ++f) {
-          check(S.ring[ring_slot(g)][f][jk] == P(self, f, HS + g, HS + jk / IC, HS + jk % IC),
+          check(S.ring[ring_slot(g)][f][jk] == P(self, f, HS + x0 + g, HS + jk / IC, HS + jk % IC),
                 "Uin value", g, jk, f);
-          check(S.u0[g % BU][f][jk] == P(self, f, HS + g, HS + jk / IC, HS + jk % IC),
+          check(S.u0[g % BU][f][jk] == P(self, f, HS + x0 + g, HS + jk / IC, HS + jk % IC),
                 "U0 value", g, jk, f);
         }
         covered_u[g][jk]++;
@@ -243,14 +255,14 @@ int main(int argc, char **argv) {
       }
       cnt_u[g]++;
       release_plane(g);
-      if (--S.reads_u[g] == 0 && g + BU < IC) issue_u0(g + BU);
+      if (--S.reads_u[g] == 0 && g + BU < NX) issue_u0(g + BU);
     } else {
       check(false, "task past the stream", pos, 0, 0);
     }
   }
-  for (int a = 0; a <= IC; ++a)
+  for (int a = 0; a <= NX; ++a)
     for (int x = 0; x < PLANE; ++x) check(covered_x[a][x] == 1, "x face coverage", a, x, 0);
-  for (int g = 0; g < IC; ++g) {
+  for (int g = 0; g < NX; ++g) {
     for (int x = 0; x < FACE_ROW * IC; ++x) {
       check(covered_y[g][x] == 1, "y face coverage", g, x, 0);
       check(covered_z[g][x] == 1, "z face coverage", g, x, 0);
@@ -262,7 +274,7 @@ int main(int argc, char **argv) {
     check(S.reads[q] == 0, "plane reads left", q - 3, S.reads[q], 0);
     check(plane_loaded[q] == (S.reads0[q] > 0), "plane loaded iff read", q - 3, 0, 0);
   }
-  for (int g = 0; g < IC; ++g)
+  for (int g = 0; g < NX; ++g)
     check(halo_loaded[g] && u0_loaded[g], "halo / U0 load", g, 0, 0);
   if (fail_count) {
     std::printf("%d failures\n", fail_count);
