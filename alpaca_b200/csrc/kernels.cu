@@ -1,12 +1,9 @@
-// Block kernels of the ALPACA right-hand side and SSP-RK3 stage update on sm_100a.
-//
-// Data stays in the reference's block layout (layout.cuh). One launch per sweep
-// direction computes the face fluxes of all work items (thread per face, the
-// 6-cell stencil read through L1), one launch applies the flux divergence and
-// the RK3 stage, one launch refreshes the face halos from neighbour interiors.
+// Block kernels beside the face fluxes (face_flux.cu, sweep.cu, ext_*.cu, pencil.cu):
+// flux divergence, stage updates, halo fill, prime states, signal speed, time-step
+// and commit records, initial conditions, interior copies. Data stays in the
+// reference's block layout (layout.cuh).
 #include <cfloat>
 #include <cstdio>
-
 
 #include "face_kernels.cuh"
 
@@ -91,8 +88,8 @@ rk_stage_rhs_kernel(double *__restrict__ U, double *__restrict__ U0,
   int const c = G::cell(i + G::fic(0), j + G::fic(1), k + G::fic(2));
   RkStage const rk = rk_stage(stage, dt);
   size_t const base = (size_t)slot * G::BLOCK_DOUBLES + c;
-  // every load before the first store (the buffers may alias, as far as the
-  // compiler knows)
+  // every load before the first store, so that a thread's loads are in flight
+  // together
   double u[G::NE], u0[G::NE], r[G::NE];
 #pragma unroll
   for (int f = 0; f < G::NE; ++f) {

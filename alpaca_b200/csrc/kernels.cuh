@@ -1,4 +1,5 @@
-// Launch interface of the block kernels (implemented in kernels.cu).
+// Launch interface of the block kernels (kernels.cu), the face fluxes (face_flux.cu,
+// sweep.cu, pencil.cu) and the small-list steps (small.cu).
 #pragma once
 
 #include <cuda_runtime.h>

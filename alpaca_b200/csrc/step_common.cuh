@@ -1,6 +1,6 @@
 // Stage-update, signal-speed and time-step arithmetic shared by every stepping
-// kernel (kernels.cu, tile_step.cu): one definition of each expression, so the
-// fused tile kernel and the face-flux + stage-update kernels round alike.
+// kernel (kernels.cu, sweep.cuh, small.cu, pencil.cu, levels.cu, tile_step.cuh): one
+// definition of each expression, so that they round alike.
 #pragma once
 
 #include <cfloat>

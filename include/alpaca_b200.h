@@ -58,8 +58,8 @@ enum {
  * stages) in the engine and serving forms (alp_rk3_stage and multi-level
  * cases: RK3). WENO5 + Hllc +
  * Einfeldt and WENO5 + Roe are the compiled fast path (FP64 and FP32_FLUX,
- * pencil sweeps); the other choices run through one FP64 face kernel that
- * selects them at run time. GlobalLaxFriedrichs takes the largest |u - c|,
+ * pencil sweeps); the other choices run through FP64 face kernels, one per
+ * stencil, that select the rest at run time. GlobalLaxFriedrichs takes the largest |u - c|,
  * |u|, |u + c| of the x velocity over all interior cells before every flux
  * evaluation and uses them in every direction, as the reference does
  * (modular_algorithm_assembler.cpp:957-985, eigendecomposition.h:457-460):
