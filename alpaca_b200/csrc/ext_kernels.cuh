@@ -12,11 +12,18 @@ namespace {
 // WENO7 reads 8-cell stencils (i-3 .. i+4), the others 6 cells (i-2 .. i+3).
 __host__ __device__ constexpr int ext_width(int st) { return st == ST_WENO7 ? 8 : 6; }
 // CTAs of 128 threads per SM (168 registers at 3); the 8-cell stencils hold a
-// third more state.
-__host__ __device__ constexpr int ext_ctas(int st) { return st == ST_WENO7 ? 2 : 3; }
+// third more state. In 1D the state is three fields: 5 CTAs (96 registers), and 4
+// for flux splitting and the 8-cell stencils. Step of 20,000 1D blocks in us, at the
+// 2 or 3 CTAs of the other dimensions against 4 or 5: WENO7 FV char 734 / 301, Roe-M
+// 745 / 330, WENO5-Z 312 / 217, HLL 259 / 223, LLF 320 / 251; 600 blocks 45 / 35, 49 /
+// 41, 33 / 29, 35 / 29, 33 / 33.
+__host__ __device__ constexpr int ext_ctas(int dim, int scheme, int st) {
+  if (dim == 1) return st == ST_WENO7 || scheme == FS_ROE ? 4 : 5;
+  return st == ST_WENO7 ? 2 : 3;
+}
 
 template <int DIM, int SCHEME, int ST, bool ACCUM>
-__global__ void __launch_bounds__(128, ext_ctas(ST))
+__global__ void __launch_bounds__(128, ext_ctas(DIM, SCHEME, ST))
 face_flux_ext_kernel(double const *__restrict__ U, int const *__restrict__ work,
                      BlockMeta const *__restrict__ meta, BlockMeta def, FluxPtrs F, long long stride,
                      int chunks, ExtPolicy<ST> pol0, unsigned long long const *__restrict__ glf) {
@@ -41,7 +48,7 @@ face_flux_ext_kernel(double const *__restrict__ U, int const *__restrict__ work,
 }
 
 template <int DIM, int SCHEME, int ST>
-__global__ void __launch_bounds__(128, ext_ctas(ST))
+__global__ void __launch_bounds__(128, ext_ctas(DIM, SCHEME, ST))
 face_flux_all_ext_kernel(double const *__restrict__ U, int const *__restrict__ work,
                          BlockMeta const *__restrict__ meta, int const *__restrict__ nbr26,
                          CaseState const *__restrict__ cases, double *__restrict__ F,
@@ -71,7 +78,8 @@ face_flux_all_ext_kernel(double const *__restrict__ U, int const *__restrict__ w
 }
 
 template <int DIM, int SCHEME, int ST>
-__global__ void __launch_bounds__(32 * kSweepWarps, ext_ctas(ST) * 4 / kSweepWarps)
+__global__ void
+__launch_bounds__(32 * kSweepWarps, ext_ctas(DIM, SCHEME, ST) * 4 / kSweepWarps)
 sweep_update_ext_kernel(double const *Uin, double const *U0, double *Uout,
                         int const *__restrict__ work, BlockMeta const *__restrict__ meta,
                         int const *__restrict__ nbr26, CaseState const *__restrict__ cases,

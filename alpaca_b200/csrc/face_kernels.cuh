@@ -44,12 +44,13 @@ template <int DIM, int DIR> struct FaceMap {
 // blocks 0.262 against 0.289 at 4. The sweeps (sweep.cuh) hold the stage
 // update's state as well: flux splitting runs them at 3. FP32-flux
 // instantiations hold fewer live doubles: FS 4 (2.05 ms vs 3: 2.23, when
-// measured), FV char 5 (1.56 vs 4: 1.64), FV prim 5 (1.455 vs 6: 1.48).
+// measured; 1D 6, 20,000 blocks 0.211 vs 4: 0.266, 600: 26.8 us vs 30.9), FV char 5
+// (1.56 vs 4: 1.64), FV prim 5 (1.455 vs 6: 1.48).
 template <int DIM, int SCHEME, typename T = double> struct FaceOccupancy {
   static constexpr bool f32 = sizeof(T) == 4;
   static constexpr int min_ctas = SCHEME == FV_CHAR ? (f32 || DIM == 2 ? 5 : 4)
                                   : SCHEME == FV_PRIM ? 5
-                                                      : 4;
+                                                      : (f32 && DIM == 1 ? 6 : 4);
   static constexpr int sweep_ctas = SCHEME == FS_ROE && !f32 ? 3 : min_ctas;
 };
 
