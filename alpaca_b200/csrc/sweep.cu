@@ -50,7 +50,7 @@ cudaError_t sweep_t(Launch const &L, double const *U0, double *Uout, double cons
 }  // namespace
 
 // Lines per warp: the longest sweep of 32, 16 or 8 that leaves three times as
-// many warps as fit on the chip (16 per SM). Short sweeps repeat the pass of the
+// many warps as fit on the chip (148 SMs of a B200, 16 warps of FV char on each). Short sweeps repeat the pass of the
 // lines' last faces more often (rows / 2 + 1 passes for rows / 2 + rows / 32 of
 // work), long ones end in a nearly empty last wave: 512 blocks 1.174 ms per
 // step at 16 lines, 8: 1.196, 32: 1.222; 2D 2025 blocks 0.235 at 8, 16: 0.241,
@@ -63,11 +63,25 @@ int sweep_rows(int dim, int nwork) {
 }
 
 // Below these counts the sweeps leave the chip idle (a warp makes five passes
-// one after the other where the face launch has five warps). Step of FV char in
-// ms, face launch + update against sweep: 64 blocks 0.174 / 0.183, 100: 0.271 /
-// 0.273, 125: 0.342 / 0.325, 216: 0.581 / 0.536, 512: 1.331 / 1.181 (100 blocks
-// of FV prim 0.251 / 0.267, flux splitting 0.300 / 0.307); 2D 529 blocks 0.074 /
-// 0.086, 1024: 0.125 / 0.129, 2025: 0.257 / 0.230.
+// one after the other where the face launch has five warps). One line for all
+// schemes, a little above where most cross. Step in us, face launch + update against
+// sweep:
+//   3D               100          112          125          144          512 blocks
+//   FV char       265 / 264    301 / 293    335 / 316    380 / 357   1352 / 1218
+//   FV prim       244 / 255    278 / 278    308 / 302    346 / 334   1230 / 1129
+//   FS Roe        296 / 300    339 / 338    373 / 362    421 / 407   1466 / 1354
+//   FV char FP32  240 / 252    275 / 275    305 / 297    344 / 333   1210 / 1070
+//   FS Roe FP32   283 / 271    321 / 299    356 / 323    403 / 363   1391 / 1218
+//   WENO5-Z       305 / 313    350 / 357    389 / 384    447 / 429   1585 / 1413
+//   WENO7         554 / 588    623 / 660    693 / 710    787 / 802   2725 / 2614
+//   2D              1024         1190         1225         1600        4096 blocks
+//   FV char       127 / 129    146 / 149    154 / 155    202 / 193    547 / 436
+//   FV prim       123 / 119    140 / 135    145 / 139    195 / 178    529 / 404
+//   FS Roe        137 / 145    158 / 164    165 / 170    224 / 209    608 / 502
+//   FV char FP32  121 / 113    139 / 129    147 / 136    195 / 178    533 / 405
+//   WENO5-Z       164 / 158    188 / 177    198 / 184    265 / 229    729 / 569
+//   WENO7         275 / 260    321 / 316    334 / 322    444 / 402   1207 / 1007
+// WENO7 crosses near 200 3D blocks and FS Roe near 1300 2D blocks: 2-3 % lost there.
 bool sweep_pays(int dim, int nwork) { return dim > 1 && nwork >= (dim == 3 ? 128 : 1200); }
 
 cudaError_t launch_sweep_update(Launch const &L, double const *U0, double *Uout, double const *F,
