@@ -50,11 +50,11 @@ cudaError_t sweep_t(Launch const &L, double const *U0, double *Uout, double cons
 }  // namespace
 
 // Lines per warp: the longest sweep of 32, 16 or 8 that leaves three times as
-// many warps as fit on the chip (148 SMs of a B200, 16 warps of FV char on each). Short sweeps repeat the pass of the
-// lines' last faces more often (rows / 2 + 1 passes for rows / 2 + rows / 32 of
-// work), long ones end in a nearly empty last wave: 512 blocks 1.174 ms per
-// step at 16 lines, 8: 1.196, 32: 1.222; 2D 2025 blocks 0.235 at 8, 16: 0.241,
-// 4: 0.247.
+// many warps as fit on the chip (148 SMs of a B200, 16 warps of FV char on each).
+// Short sweeps repeat the pass of the lines' last faces more often (rows / 2 + 1
+// passes for rows / 2 + rows / 32 of work), long ones end in a nearly empty last
+// wave: 512 blocks 1.174 ms per step at 16 lines, 8: 1.196, 32: 1.222; 2D 2025 blocks
+// 0.235 at 8, 16: 0.241, 4: 0.247.
 int sweep_rows(int dim, int nwork) {
   int const lines = dim == 3 ? IC * IC : IC;
   int rows = dim == 3 ? 32 : 16;
