@@ -223,7 +223,8 @@ def reference_programs():
     return out
 
 
-@pytest.mark.skipif(not os.path.isdir(REF), reason="reference input files not present")
+@pytest.mark.skipif(not glob.glob(os.path.join(REF, "**", "*.xml"), recursive=True),
+                    reason="reference input files not present")
 def test_every_reference_initial_condition_compiles_and_agrees():
     progs = reference_programs()
     assert len(progs) >= 40
